@@ -109,6 +109,12 @@ __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P
     }
 }
 
+// Six blocks of 128 threads per SM for the batch's group pass: a group keeps
+// its own scene's pointers in registers.
+#ifndef GRIDRT_GROUP_BATCH_MIN_BLOCKS
+#define GRIDRT_GROUP_BATCH_MIN_BLOCKS 6
+#endif
+
 // Many (scene, ray batch) tasks in one persistent launch.  Task t owns the
 // 32-aligned index range [first, first + n) of one flattened ray space, so a
 // 32-ray claim always falls inside one task: scene and mode are warp-uniform.
@@ -163,60 +169,62 @@ __global__ void __launch_bounds__(128, GRIDRT_TRACE_MIN_BLOCKS)
     }
 }
 
-// Warp-per-ray pass over the rays a batch launch deferred (flattened
-// indices); each group resolves its own task, scene and mode.
+// Group pass over the rays a batch launch deferred (flattened indices); each
+// group resolves its own task, scene and mode.
 template <int G>
-__global__ void __launch_bounds__(128) trace_wide_batch_kernel(const BatchScene* __restrict__ scenes, int nscenes,
-                                                               const BatchTask* __restrict__ tasks, int ntasks,
-                                                               unsigned long long* counter,
-                                                               const int2* __restrict__ defer, int32_t defer_cap) {
+__global__ void __launch_bounds__(128, GRIDRT_GROUP_BATCH_MIN_BLOCKS)
+    trace_group_batch_kernel(const BatchScene* __restrict__ scenes, int nscenes, const BatchTask* __restrict__ tasks,
+                             int ntasks, unsigned long long* counter, const int2* __restrict__ defer,
+                             int32_t defer_cap) {
     pdl_begin();
     __shared__ SParams P[kMaxBatchScenes];
     for (int i = threadIdx.x; i < nscenes; i += blockDim.x) fill_sparams(scenes[i].view.params, P[i]);
     __syncthreads();
-    const int lane = threadIdx.x & 31, gl = lane & (G - 1), grp = lane / G;
-    unsigned long long nd = counter[1];
-    if (nd > (unsigned long long)defer_cap) nd = (unsigned long long)defer_cap;
-    uint32_t cells = 0, tests = 0;
+    const int gl = threadIdx.x & (G - 1);
+    constexpr int kWant = G < 32 ? 16 / G : 1;
+    unsigned long long total = counter[1];
+    if (total > (unsigned long long)defer_cap) total = (unsigned long long)defer_cap;
+    bool busy = false, exhausted = false, any = false;
+    int todo = 0, scene = 0;
+    int3 sg = make_int3(0, 0, 0);
+    Lane L = idle_lane();
+    TraceIO io{};
     for (;;) {
-        unsigned long long j0 = 0;
-        if (lane == 0) j0 = atomicAdd(counter + 2, (unsigned long long)(32 / G));
-        j0 = __shfl_sync(FULL, j0, 0);
-        if (j0 >= nd) break;
-        const unsigned long long j = j0 + grp;
-        const bool valid = j < nd;
-        bool done = true, any = false;
-        int scene = 0;
-        Lane L;
-        L.best = kFltMax;
-        L.id = -1;
-        TraceIO io{};
-        if (valid) {
-            const int2 d = __ldg(defer + j);
-            const BatchTask T = tasks[find_task(tasks, ntasks, (long long)d.x)];
-            scene = T.scene;
-            any = T.mode == MODE_ANY;
-            io.rays = T.rays;
-            io.n = T.n;
-            L.ray = (int32_t)((long long)d.x - T.first);
-            if (any) {
+        const unsigned idle = __ballot_sync(FULL, !busy);
+        if (!exhausted && __popc(idle) >= kWant * G) {
+            const unsigned long long r = claim_groups<G>(idle, counter + 2, total, exhausted);
+            if (!busy && r < total) {
+                const int2 d = __ldg(defer + r);
+                const BatchTask T = tasks[find_task(tasks, ntasks, (long long)d.x)];
+                scene = T.scene;
+                any = T.mode == MODE_ANY;
+                io.rays = T.rays;
                 io.occ = static_cast<uint8_t*>(T.out);
-                done = !start_ray<MODE_ANY>(P[scene], io, L, L.ray);
-            } else {
                 io.hits = static_cast<int4*>(T.out);
-                done = !start_ray<MODE_NEAREST>(P[scene], io, L, L.ray);
-            }
-            if (done) {
-                if (L.id != -2) L.id = -1;
-            } else {
-                resume_at(P[scene], L, d.y);
+                L.ray = (int32_t)((long long)d.x - T.first);
+                busy = any ? start_ray<MODE_ANY>(P[scene], io, L, L.ray) : start_ray<MODE_NEAREST>(P[scene], io, L, L.ray);
+                if (busy) {
+                    resume_at(P[scene], L, d.y);
+                } else {
+                    if (L.id != -2) L.id = -1;
+                    if (any) finish_ray<MODE_ANY>(io, P[scene], scenes[scene].view, L, gl == 0);
+                    else finish_ray<MODE_NEAREST>(io, P[scene], scenes[scene].view, L, gl == 0);
+                }
+                todo = gl;
+                sg = step_signs(L);
             }
         }
+        if (!__any_sync(FULL, busy)) {
+            if (exhausted) break;
+            continue;
+        }
         const SceneView V = scenes[scene].view;
-        wide_walk<G>(P[scene], V, L, done, any, cells, tests);
-        if (valid && gl == 0) {
-            if (any) finish_ray<MODE_ANY>(io, P[scene], V, L);
-            else finish_ray<MODE_NEAREST>(io, P[scene], V, L);
+        const GroupOut r = group_batch<G>(P[scene], V, L, sg, busy, any, busy ? todo : 0, kNoHeavy);
+        todo = G;
+        if (busy && r.step == GROUP_DONE) {
+            if (any) finish_ray<MODE_ANY>(io, P[scene], V, L, gl == 0);
+            else finish_ray<MODE_NEAREST>(io, P[scene], V, L, gl == 0);
+            busy = false;
         }
     }
 }
@@ -444,15 +452,15 @@ static void launch_batch_er(const BatchScene* scenes, int nscenes, const BatchTa
 }
 
 template <int G>
-static void launch_wide_batch(const BatchScene* scenes, int nscenes, const BatchTask* tasks, int ntasks,
-                              const TraceSlot& slot, int num_sms, cudaStream_t st) {
+static void launch_group_batch(const BatchScene* scenes, int nscenes, const BatchTask* tasks, int ntasks,
+                               const TraceSlot& slot, int num_sms, cudaStream_t st) {
     static int per_sm = 0;
     if (per_sm == 0) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_wide_batch_kernel<G>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_group_batch_kernel<G>, 128, 0);
         per_sm = b > 0 ? b : 1;
     }
-    launch_k(trace_wide_batch_kernel<G>, (unsigned)(per_sm * num_sms), 128, 0, st, scenes, nscenes, tasks, ntasks,
+    launch_k(trace_group_batch_kernel<G>, (unsigned)(per_sm * num_sms), 128, 0, st, scenes, nscenes, tasks, ntasks,
              slot.ctr, slot.defer, slot.defer_cap);
 }
 
@@ -469,10 +477,10 @@ void launch_trace_batch(const BatchScene* scenes, int nscenes, const BatchTask* 
     else if (tune.empty_run <= 8) launch_batch_er<8>(scenes, nscenes, tasks, ntasks, total, slot, heavy, refill_for(tune, 0), num_sms, st);
     else launch_batch_er<16>(scenes, nscenes, tasks, ntasks, total, slot, heavy, refill_for(tune, 0), num_sms, st);
     if (defer) {
-        if (tune.heavy_lanes <= 4) launch_wide_batch<4>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
-        else if (tune.heavy_lanes <= 8) launch_wide_batch<8>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
-        else if (tune.heavy_lanes <= 16) launch_wide_batch<16>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
-        else launch_wide_batch<32>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
+        if (tune.heavy_lanes <= 4) launch_group_batch<4>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
+        else if (tune.heavy_lanes <= 8) launch_group_batch<8>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
+        else if (tune.heavy_lanes <= 16) launch_group_batch<16>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
+        else launch_group_batch<32>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
     }
 }
 

@@ -36,7 +36,6 @@ namespace gridrt {
 static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the warp-per-ray pass
 static constexpr int32_t kNoHeavy = 0x7fffffff;
-static constexpr int kWideEmptyRun = 8;     // empty cells a deferred ray's group walks per turn
 // A ray is also deferred once its tests would pass kHeavyWorkMult x the
 // heavy-cell threshold in total (0: only long lists defer).
 #ifndef GRIDRT_HEAVY_WORK_MULT
@@ -803,16 +802,6 @@ __global__ void __launch_bounds__(TPB, GRIDRT_TRACE_MIN_BLOCKS * 128 / TPB) trac
     if (COUNT) flush_counters(io.ctr, started, cells, tests);
 }
 
-// Warp-per-ray pass over the deferred rays, G lanes per ray (32/G rays a
-// warp): the G lanes of a group hold the same ray and walk the same cells; a
-// cell's list is split over them (lane j of the group tests entries j, j+G,
-// ...), each lane keeping the first minimum of its share, and the group
-// takes the minimum t, ties to the smaller triangle id.  Lists are sorted by
-// id, so that is the first minimum in list order: the one-lane walk's result.
-// ANY rays are occluded when that minimum is below tmax -- also the one-lane
-// walk's rule, which accepts every new minimum and stops at the first below
-// tmax.
-//
 // A deferred ray resumes at the cell where its lane stopped: every coordinate
 // moved monotonically from the start cell, one step per crossing of its
 // axis, each adding tD to tM, so replaying those additions in order rebuilds
@@ -830,187 +819,288 @@ __device__ __forceinline__ void resume_at(const SParams& P, Lane& L, int32_t cel
     L.budget -= sx + sy + sz;
 }
 
-// Walks the group's ray (state in L, identical on its G lanes) to its end.
-// Every lane of the warp calls it; groups that are done idle through the
-// warp-wide list loop and reductions.
-// With `huge` set, a group whose ray reaches a list above kHugeList queues
-// {huge_tag, cell} for the block-per-ray pass instead (counted there) and
-// returns true: that pass finishes the ray.
+// ---------------------------------------------------------------------------
+// Group walk: G lanes trace one ray together, lane j at the j-th next cell of
+// its walk.  Used for the rays the one-lane walk defers (a long list, or many
+// tests made already) and for every ray of a launch with RTG_TUNE_LANES 2 or 4.
+//
+// Bound by latency: a walk is a chain of dependent loads (occupancy word, list
+// bounds, ids, records) of ~1 us a non-empty cell, and a launch ends with its
+// longest rays.  Lanes that split one cell's list at a time shorten only long
+// lists; most of a long ray's cells hold two or three triangles.  So the lanes
+// take G consecutive cells at once: each steps the whole DDA itself (the same
+// additions in the same order, ten instructions a cell and no loads), their G
+// cells' loads are in flight together, and the lists found, end to end, are
+// dealt out evenly over the lanes.  The lane that owns an entry's cell gives it
+// the list position and the cell's window by shuffle.  A hit in an earlier cell
+// beats any in a later one; inside a cell the smaller t wins, then the smaller
+// id (ids ascend along a list), which is the one-lane walk's result.
+// The pass over deferred rays alone, before -> after: 215 -> 75 us behind 1.5 M
+// random rays in 495,000 triangles, 70 -> 46 us behind a 1024^2 frame of the
+// 102,400-triangle sphere.
+// ---------------------------------------------------------------------------
+// What a batch of G cells came to: the ray goes on, is finished (L.id), or
+// stopped before a list longer than `thr` (its cell and length).
+enum GroupStep : int { GROUP_ON = 0, GROUP_DONE = 1, GROUP_LIST = 2 };
+struct GroupOut {
+    int step;
+    int32_t cell, len;        // GROUP_LIST
+    int32_t cells, tests;     // visited and tested by the one-lane walk's count
+};
+
+// Direction of a DDA step along each axis (vr::sign of the direction).
+__device__ __forceinline__ int3 step_signs(const Lane& L) {
+    return make_int3(L.dx < 0.0f ? -1 : (L.dx > 0.0f ? 1 : 0), L.dy < 0.0f ? -1 : (L.dy > 0.0f ? 1 : 0),
+                     L.dz < 0.0f ? -1 : (L.dz > 0.0f ? 1 : 0));
+}
+
+// Moves every lane `todo` cells on (its place in the group for a new ray, G
+// after that, 0 to visit the same cells again) and tests the lists of the
+// group's cells.  Called by the whole warp; `busy` is the same for a group.
 template <int G>
-__device__ __forceinline__ bool wide_walk(const SParams& P, const SceneView& s, Lane& L, bool done, bool any,
-                                          uint32_t& cells, uint32_t& tests, int2* huge = nullptr,
-                                          int32_t huge_cap = 0, unsigned long long* huge_ctr = nullptr,
-                                          int32_t huge_tag = 0) {
-    const int gl = threadIdx.x & (G - 1);
-    bool handed = false;
-    const int32_t nx = P.res[0], nxy = P.res[0] * P.res[1];
-    while (__any_sync(FULL, !done)) {
-        int32_t b = 0, e = 0;
-        float hi = 0.0f;
-        if (!done) {
-            // up to kWideEmptyRun empty cells per turn before a list (as the
-            // one-lane walk does), so empty stretches skip the list and
-            // reduction steps below
-            for (int r = 0; r < kWideEmptyRun; ++r) {
-                if (gl == 0) ++cells;
-                const int32_t w = (L.x >> 2) + (L.y >> 2) * P.bx + (L.z >> 1) * P.bxby;
-                if (__ldg(s.occ + w) & occ_bit(L.x, L.y, L.z)) {
-                    const int32_t c = L.x + L.y * nx + L.z * nxy;
-                    b = __ldg(s.offsets + c);
-                    e = __ldg(s.offsets + c + 1);
-                    hi = fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon);
-                    break;
+__device__ __forceinline__ GroupOut group_batch(const SParams& P, const SceneView& s, Lane& L, const int3& sg,
+                                                bool busy, bool any, int todo, int32_t thr) {
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
+    constexpr unsigned gm = G == 32 ? FULL : ((1u << G) - 1u);
+    // dda_step without its exit test: a coordinate that has left the grid
+    // moves on outward, so the batch's end tells whether it ever left
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+        const bool go = j < todo;
+        const bool ax = L.tMx < L.tMy && L.tMx < L.tMz;
+        const bool ay = !ax && L.tMy < L.tMz;
+        if (go && ax) { L.x += sg.x; L.tMx = fadd(L.tMx, L.tDx); }
+        if (go && ay) { L.y += sg.y; L.tMy = fadd(L.tMy, L.tDy); }
+        if (go && !ax && !ay) { L.z += sg.z; L.tMz = fadd(L.tMz, L.tDz); }
+    }
+    L.budget -= todo;
+    const bool out = (unsigned)L.x >= (unsigned)P.res[0] || (unsigned)L.y >= (unsigned)P.res[1] ||
+                     (unsigned)L.z >= (unsigned)P.res[2] || L.budget <= 0;
+    int32_t b = 0, n = 0, c = 0;
+    if (busy && !out) {
+        const int32_t w = (L.x >> 2) + (L.y >> 2) * P.bx + (L.z >> 1) * P.bxby;
+        if (__ldg(s.occ + w) & occ_bit(L.x, L.y, L.z)) {
+            c = L.x + P.res[0] * (L.y + L.z * P.res[1]);
+            b = __ldg(s.offsets + c);
+            n = __ldg(s.offsets + c + 1) - b;
+        }
+    }
+    const unsigned om = (__ballot_sync(FULL, busy && out) >> g0) & gm;   // lanes past the grid
+    int hj = G;                                                          // cell of this lane's hit
+    int fh = G;                                                          // first cell with a list above thr
+    int32_t limit = 0, incl = n;
+    if (__any_sync(FULL, n > 0)) {
+        const float hi = fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon);
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const int32_t y = __shfl_up_sync(FULL, incl, o, G);
+            if (gl >= o) incl += y;
+        }
+        const int32_t excl = incl - n, first = b - excl;
+        const unsigned hm = (__ballot_sync(FULL, n > thr) >> g0) & gm;
+        if (hm) fh = __ffs(hm) - 1;
+        limit = __shfl_sync(FULL, hm ? excl : incl, hm ? fh : G - 1, G);   // hm is the same for the group
+        for (int32_t base = 0; __any_sync(FULL, base < limit); base += G) {
+            const int32_t q = base + gl;
+            int j = 0;                               // the lane whose list holds entry q
+#pragma unroll
+            for (int w = G >> 1; w > 0; w >>= 1)
+                if (__shfl_sync(FULL, incl, j + w - 1, G) <= q) j += w;
+            const int32_t at = __shfl_sync(FULL, first, j, G) + q;
+            const float hij = __shfl_sync(FULL, hi, j, G);
+            if (q < limit && j <= hj) {
+                int32_t t;
+                float4 A, B, C;
+                if (s.crec) {
+                    A = __ldg(s.crec + 3 * (int64_t)at);
+                    B = __ldg(s.crec + 3 * (int64_t)at + 1);
+                    C = __ldg(s.crec + 3 * (int64_t)at + 2);
+                    t = __float_as_int(A.w);
+                } else {
+                    t = __ldg(s.ids + at);
+                    A = __ldg(s.tris + 3 * (int64_t)t);
+                    B = __ldg(s.tris + 3 * (int64_t)t + 1);
+                    C = __ldg(s.tris + 3 * (int64_t)t + 2);
                 }
-                if (dda_step(P, L)) {
-                    L.id = -1;
-                    done = true;
-                    break;
-                }
+                const int32_t was = L.id;
+                test_tri<MODE_NEAREST>(L, t, A, B, C, hij, s.wald);
+                if (L.id != was) hj = j;
+            }
+            if (__any_sync(FULL, hj < G)) {          // nothing after a hit's cell is needed
+                int m = hj;
+#pragma unroll
+                for (int o = G >> 1; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(FULL, m, o));
+                const int32_t end = __shfl_sync(FULL, incl, m & (G - 1), G);
+                if (m < G) limit = min(limit, end);
             }
         }
-        if (huge) {
-            // lists above kHugeList go to the block-per-ray pass (which visits
-            // the cell again), while its queue has room
-            const bool want = !done && e - b > kHugeList;
-            if (__ballot_sync(FULL, want)) {
-                unsigned long long at = 0;
-                if (want && gl == 0) at = atomicAdd(huge_ctr, 1ull);
-                at = __shfl_sync(FULL, at, (int)(threadIdx.x & 31) & ~(G - 1));
-                if (want && at < (unsigned long long)huge_cap) {
-                    if (gl == 0) {
-                        // longest first: lists of kHugeLong+ entries fill the
-                        // queue from its back (huge_ctr[2] of them), the rest
-                        // from its front (huge_ctr[3]); together they number
-                        // the reservations that fit, so the two never meet
-                        const bool longl = e - b >= kHugeLong;
-                        const unsigned long long pos = atomicAdd(huge_ctr + (longl ? 2 : 3), 1ull);
-                        huge[longl ? (unsigned long long)huge_cap - 1 - pos : pos] =
-                            make_int2(huge_tag, L.x + L.y * nx + L.z * nxy);
-                        --cells;
-                    }
-                    handed = done = true;
-                    b = e = 0;
-                }
-            }
-        }
-        if (gl == 0) tests += (uint32_t)(e - b);
-        const unsigned trips = __reduce_max_sync(FULL, (unsigned)((e - b + G - 1) / G));
-        if (trips == 0) continue;   // no group of the warp is at a list this turn
-        // two entries per lane and turn, both loaded before either is tested
-        for (unsigned it = 0; it < trips; it += 2) {
-            const int32_t i0 = b + gl + (int32_t)it * G, i1 = i0 + G;
-            int32_t t0 = -1, t1 = -1;
-            float4 A0, B0, C0, A1, B1, C1;
-            if (s.crec) {
-                if (i0 < e) {
-                    A0 = __ldg(s.crec + 3 * (int64_t)i0);
-                    B0 = __ldg(s.crec + 3 * (int64_t)i0 + 1);
-                    C0 = __ldg(s.crec + 3 * (int64_t)i0 + 2);
-                    t0 = __float_as_int(A0.w);
-                }
-                if (i1 < e) {
-                    A1 = __ldg(s.crec + 3 * (int64_t)i1);
-                    B1 = __ldg(s.crec + 3 * (int64_t)i1 + 1);
-                    C1 = __ldg(s.crec + 3 * (int64_t)i1 + 2);
-                    t1 = __float_as_int(A1.w);
-                }
-            } else {
-                if (i0 < e) t0 = __ldg(s.ids + i0);
-                if (i1 < e) t1 = __ldg(s.ids + i1);
-                if (t0 >= 0) {
-                    A0 = __ldg(s.tris + 3 * (int64_t)t0);
-                    B0 = __ldg(s.tris + 3 * (int64_t)t0 + 1);
-                    C0 = __ldg(s.tris + 3 * (int64_t)t0 + 2);
-                }
-                if (t1 >= 0) {
-                    A1 = __ldg(s.tris + 3 * (int64_t)t1);
-                    B1 = __ldg(s.tris + 3 * (int64_t)t1 + 1);
-                    C1 = __ldg(s.tris + 3 * (int64_t)t1 + 2);
-                }
-            }
-            if (t0 >= 0) test_tri<MODE_NEAREST>(L, t0, A0, B0, C0, hi, s.wald);
-            if (t1 >= 0) test_tri<MODE_NEAREST>(L, t1, A1, B1, C1, hi, s.wald);
-        }
+    }
+    if (__any_sync(FULL, hj < G)) {
 #pragma unroll
         for (int o = G >> 1; o > 0; o >>= 1) {
+            const int oj = __shfl_xor_sync(FULL, hj, o);
             const float ot = __shfl_xor_sync(FULL, L.best, o);
             const int32_t oid = __shfl_xor_sync(FULL, L.id, o);
-            if (ot < L.best || (ot == L.best && (uint32_t)oid < (uint32_t)L.id)) {
+            if (oj < hj || (oj == hj && (ot < L.best || (ot == L.best && (uint32_t)oid < (uint32_t)L.id)))) {
+                hj = oj;
                 L.best = ot;
                 L.id = oid;
             }
         }
-        if (!done && e > b) {   // groups that tested a list this turn
-            if (L.best < kFltMax) {
-                if (any && !(L.best < L.tmax)) L.id = -1;
-                done = true;
-            } else if (dda_step(P, L)) {
-                L.id = -1;
-                done = true;
-            }
-        }
     }
-    return handed;
+    // the last shuffles of the batch: the groups part ways below
+    const int32_t hit_tests = __shfl_sync(FULL, incl, hj & (G - 1), G);
+    GroupOut r;
+    r.cell = __shfl_sync(FULL, c, fh & (G - 1), G);
+    r.len = __shfl_sync(FULL, n, fh & (G - 1), G);
+    r.tests = limit;
+    if (hj < G) {
+        r.step = GROUP_DONE;
+        r.cells = hj + 1;
+        r.tests = hit_tests;
+        if (any && !(L.best < L.tmax)) L.id = -1;   // any-hit: the first cell with a hit decides
+    } else if (fh < G) {
+        r.step = GROUP_LIST;
+        r.cells = fh;
+    } else if (om) {
+        r.step = GROUP_DONE;
+        r.cells = __ffs(om) - 1;
+        L.id = -1;
+    } else {
+        r.step = GROUP_ON;
+        r.cells = G;
+    }
+    return r;
 }
 
-// Five blocks of 128 threads per SM (at most 102 registers a thread): the
-// exact decisions' code took the group pass from 96 to 109 registers, four
-// blocks an SM, and 20% longer.
-#ifndef GRIDRT_WIDE_MIN_BLOCKS
-#define GRIDRT_WIDE_MIN_BLOCKS 5
+// A lane without a ray, defined so that the warp can step it idly.
+__device__ __forceinline__ Lane idle_lane() {
+    Lane L;
+    L.ox = L.oy = L.oz = L.dx = L.dy = L.dz = 0.0f;
+    L.tMx = L.tMy = L.tMz = L.tDx = L.tDy = L.tDz = 0.0f;
+    L.x = L.y = L.z = 0;
+    L.budget = 0;
+    L.tmax = L.lo = 0.0f;
+    L.best = kFltMax;
+    L.id = -1;
+    L.ray = 0;
+    return L;
+}
+
+// The next rays for a warp's idle groups: `want` of them claimed with one
+// atomicAdd on *counter, handed out in group order.  Sets `exhausted` once the
+// claims pass `total`.
+template <int G>
+__device__ __forceinline__ unsigned long long claim_groups(unsigned idle, unsigned long long* counter,
+                                                           unsigned long long total, bool& exhausted) {
+    const int lane = threadIdx.x & 31;
+    const unsigned want = (unsigned)__popc(idle) / G;
+    unsigned long long r = 0;
+    if (lane == 0) r = atomicAdd(counter, (unsigned long long)want);
+    r = __shfl_sync(FULL, r, 0);
+    if (r + want >= total) exhausted = true;
+    return r + (unsigned)__popc(idle & ((1u << (lane & ~(G - 1))) - 1u)) / G;
+}
+
+// Eight blocks of 128 threads per SM: six (80 registers) made the group walk
+// of 4 M random rays 9% slower.
+#ifndef GRIDRT_GROUP_MIN_BLOCKS
+#define GRIDRT_GROUP_MIN_BLOCKS 8
 #endif
-template <int MODE, bool COUNT, int G>
-__global__ void __launch_bounds__(128, GRIDRT_WIDE_MIN_BLOCKS) trace_wide_kernel(SceneView s, TraceIO io) {
+
+// QUEUE: the rays another pass deferred, from the cell it stopped at; else the
+// launch's rays from their start.  Idle groups take new rays once half of the
+// warp's groups are idle.  A ray that comes to a long list is handed on, while
+// there is room, to the pass that resumes it there (and counts that cell): from
+// the start (io.defer set) lists above io.heavy to the deferred pass, else
+// lists above kHugeList to the block-per-ray pass.
+template <int MODE, bool COUNT, int G, bool QUEUE>
+__global__ void __launch_bounds__(128, GRIDRT_GROUP_MIN_BLOCKS) trace_group_kernel(SceneView s, TraceIO io) {
     pdl_begin();
     __shared__ SParams P;
     load_sparams(s.params, P);
-    const int lane = threadIdx.x & 31, gl = lane & (G - 1), grp = lane / G;
-    // the deferred rays, or (no queue: the group walk from the start) every ray
-    unsigned long long nd = io.defer ? io.counter[1] : (unsigned long long)io.n;
-    if (io.defer && nd > (unsigned long long)io.defer_cap) nd = (unsigned long long)io.defer_cap;
-    uint32_t cells = 0, tests = 0;
+    const int gl = threadIdx.x & (G - 1);
+    constexpr int kWant = G < 32 ? 16 / G : 1;
+    unsigned long long total = (unsigned long long)io.n;
+    if (QUEUE) {
+        total = io.counter[1];
+        if (total > (unsigned long long)io.defer_cap) total = (unsigned long long)io.defer_cap;
+    }
+    const bool to_defer = !QUEUE && io.defer;
+    const int32_t thr0 = to_defer ? io.heavy : (io.huge ? kHugeList : kNoHeavy);
+    uint32_t cells = 0, tests = 0, started = 0;
+    bool busy = false, exhausted = false;
+    int todo = 0;
+    int32_t thr = thr0;
+    int3 sg = make_int3(0, 0, 0);
+    Lane L = idle_lane();
     for (;;) {
-        unsigned long long j0 = 0;
-        if (lane == 0) j0 = atomicAdd(io.counter + 2, (unsigned long long)(32 / G));
-        j0 = __shfl_sync(FULL, j0, 0);
-        if (j0 >= nd) break;
-        const unsigned long long j = j0 + grp;
-        const bool valid = j < nd;
-        bool done = true;
-        Lane L;
-        L.best = kFltMax;
-        L.id = -1;
-        bool shadow = false;      // MODE_FRAME: the entry is a shadow ray (its slot holds it)
-        if (valid) {
-            const int2 d = io.defer ? __ldg(io.defer + j) : make_int2((int32_t)j, -1);
-            shadow = MODE == MODE_FRAME && d.x < 0;
-            L.ray = shadow ? -1 - d.x : d.x;
-            done = shadow ? !start_ray<MODE_ANY>(P, io, L, L.ray) : !start_ray<MODE>(P, io, L, L.ray);
-            if (done) {
-                if (L.id != -2) L.id = -1;
-            } else if (d.y >= 0) {
-                resume_at(P, L, d.y);
+        const unsigned idle = __ballot_sync(FULL, !busy);
+        if (!exhausted && __popc(idle) >= kWant * G) {
+            const unsigned long long r = claim_groups<G>(idle, io.counter + (QUEUE ? 2 : 0), total, exhausted);
+            if (!busy && r < total) {
+                const int2 d = QUEUE ? __ldg(io.defer + r) : make_int2((int32_t)r, -1);
+                const bool shadow = MODE == MODE_FRAME && d.x < 0;   // a frame's shadow ray (its slot holds it)
+                L.ray = shadow ? -1 - d.x : d.x;
+                busy = shadow ? start_ray<MODE_ANY>(P, io, L, L.ray) : start_ray<MODE>(P, io, L, L.ray);
+                if (!QUEUE && gl == 0) ++started;
+                if (busy) {
+                    if (QUEUE) resume_at(P, L, d.y);
+                } else {
+                    if (L.id != -2) L.id = -1;
+                    busy = finish_ray<MODE>(io, P, s, L, gl == 0);
+                }
+                todo = gl;
+                thr = thr0;
+                sg = step_signs(L);
             }
         }
-        const bool handed = wide_walk<G>(P, s, L, done, MODE == MODE_ANY || shadow, cells, tests, io.huge,
-                                         io.huge_cap, io.counter + 3, shadow ? -1 - L.ray : L.ray);
-        if (MODE == MODE_FRAME) {
+        if (!__any_sync(FULL, busy)) {
+            if (exhausted) break;
+            continue;
+        }
+        const bool any = MODE == MODE_ANY || (MODE == MODE_FRAME && L.tmax > -kFltMax);
+        GroupOut r = group_batch<G>(P, s, L, sg, busy, any, busy ? todo : 0, thr);
+        todo = G;
+        const bool hand = busy && r.step == GROUP_LIST;
+        if (__any_sync(FULL, hand)) {
+            unsigned long long at = 0;
+            if (hand && gl == 0) at = atomicAdd(io.counter + (to_defer ? 1 : 3), 1ull);
+            at = __shfl_sync(FULL, at, 0, G);
+            if (hand && at < (unsigned long long)(to_defer ? io.defer_cap : io.huge_cap)) {
+                if (to_defer) {
+                    if (gl == 0) io.defer[at] = make_int2(defer_tag<MODE>(L, io), r.cell);
+                } else if (gl == 0) {
+                    // longest first: lists of kHugeLong+ entries fill the
+                    // queue from its back (counter word 5 of them), the rest
+                    // from its front (word 6); together they number the
+                    // reservations that fit, so the two never meet
+                    const bool longl = r.len >= kHugeLong;
+                    const unsigned long long pos = atomicAdd(io.counter + (longl ? 5 : 6), 1ull);
+                    io.huge[longl ? (unsigned long long)io.huge_cap - 1 - pos : pos] =
+                        make_int2(defer_tag<MODE>(L, io), r.cell);
+                }
+                busy = false;
+            } else if (hand) {
+                thr = kNoHeavy;   // the queue is full: the group visits its cells again and tests the list
+                todo = 0;
+                r.cells = r.tests = 0;
+            }
+        }
+        if (COUNT && gl == 0 && (busy || hand)) {
+            cells += (uint32_t)r.cells;
+            tests += (uint32_t)r.tests;
+        }
+        if (busy && r.step == GROUP_DONE) {
             // a camera ray's group goes on with its hit's shadow ray: every
             // lane sets it up from the hit (one writes the results)
-            bool second = false;
-            if (valid && !handed) second = finish_ray<MODE>(io, P, s, L, gl == 0);
-            bool done2 = !second;
-            const bool handed2 = wide_walk<G>(P, s, L, done2, true, cells, tests, io.huge, io.huge_cap,
-                                              io.counter + 3, -1 - L.ray);
-            if (second && !handed2 && gl == 0) finish_ray<MODE>(io, P, s, L);
-        } else if (valid && gl == 0 && !handed) {
-            finish_ray<MODE>(io, P, s, L);
+            busy = finish_ray<MODE>(io, P, s, L, gl == 0);
+            todo = gl;
+            thr = thr0;
+            sg = step_signs(L);
         }
     }
-    if (COUNT) {
-        if (gl != 0) cells = tests = 0;
-        flush_counters(io.ctr, 0, cells, tests);
-    }
+    if (COUNT) flush_counters(io.ctr, started, cells, tests);
 }
 
 // Block-per-ray pass over the rays the group pass met at a list above
@@ -1323,24 +1413,27 @@ inline void launch_count(const SceneView& s, const TraceIO& io, const TraceTunin
     else launch_er<MODE, COUNT, 16>(s, io, tune, num_sms, st);
 }
 
-template <int MODE, bool COUNT, int G>
-inline void launch_wide_g(const SceneView& s, const TraceIO& io, int num_sms, cudaStream_t st) {
+// The group pass: as many blocks as fit on the device, or as the launch's rays
+// need.
+template <int MODE, bool COUNT, int G, bool QUEUE>
+inline void launch_group(const SceneView& s, const TraceIO& io, int num_sms, cudaStream_t st) {
     static int per_sm = 0;
     if (per_sm == 0) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_wide_kernel<MODE, COUNT, G>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_group_kernel<MODE, COUNT, G, QUEUE>, 128, 0);
         per_sm = b > 0 ? b : 1;
     }
-    launch_k(trace_wide_kernel<MODE, COUNT, G>, (unsigned)(per_sm * num_sms), 128, 0, st, s, io);
+    const long long full = (long long)per_sm * num_sms, need = (io.n + 128 / G - 1) / (128 / G);
+    launch_k(trace_group_kernel<MODE, COUNT, G, QUEUE>, (unsigned)(need < full ? need : full), 128, 0, st, s, io);
 }
 
 template <int MODE, bool COUNT>
-inline void launch_wide(const SceneView& s, const TraceIO& io, const TraceTuning& tune, int num_sms,
-                        cudaStream_t st) {
-    if (tune.heavy_lanes <= 4) launch_wide_g<MODE, COUNT, 4>(s, io, num_sms, st);
-    else if (tune.heavy_lanes <= 8) launch_wide_g<MODE, COUNT, 8>(s, io, num_sms, st);
-    else if (tune.heavy_lanes <= 16) launch_wide_g<MODE, COUNT, 16>(s, io, num_sms, st);
-    else launch_wide_g<MODE, COUNT, 32>(s, io, num_sms, st);
+inline void launch_deferred(const SceneView& s, const TraceIO& io, const TraceTuning& tune, int num_sms,
+                            cudaStream_t st) {
+    if (tune.heavy_lanes <= 4) launch_group<MODE, COUNT, 4, true>(s, io, num_sms, st);
+    else if (tune.heavy_lanes <= 8) launch_group<MODE, COUNT, 8, true>(s, io, num_sms, st);
+    else if (tune.heavy_lanes <= 16) launch_group<MODE, COUNT, 16, true>(s, io, num_sms, st);
+    else launch_group<MODE, COUNT, 32, true>(s, io, num_sms, st);
 }
 
 // As many blocks as fit on the GPU claim the queued rays: each ray's lists
@@ -1373,27 +1466,21 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
     io.huge = defer ? slot.huge : nullptr;
     io.huge_cap = io.huge ? slot.huge_cap : 0;
     cudaMemsetAsync(slot.ctr, 0, 8 * sizeof(unsigned long long), st);
-    if (tune.lanes > 1 && !io.ctr) {
-        // every ray walked by a group of lanes from its start (the group
-        // pass with no queue); lists above kHugeList are still handed to
-        // the block-per-ray pass
-        io.defer = nullptr;
-        io.defer_cap = 0;
-        io.heavy = kNoHeavy;
-        io.huge = slot.huge;
-        io.huge_cap = io.huge ? slot.huge_cap : 0;
-        count_launches(io.huge ? 2 : 1);
-        if (tune.lanes == 2) launch_wide_g<MODE, false, 2>(s, io, num_sms, st);
-        else launch_wide_g<MODE, false, 4>(s, io, num_sms, st);
-        if (io.huge) launch_huge<MODE, false>(s, io, num_sms, st);
-        return;
-    }
     count_launches(defer ? (io.huge ? 3 : 2) : 1);
-    if (io.ctr) launch_count<MODE, true>(s, io, tune, num_sms, st);
-    else launch_count<MODE, false>(s, io, tune, num_sms, st);
+    if (tune.lanes > 1 && !io.ctr) {
+        // every ray walked by a group of lanes from its start; a list that
+        // would take its lanes more than heavy_cell / 2 turns is deferred
+        if (defer && io.heavy < kNoHeavy / 4) io.heavy = io.heavy * tune.lanes / 2;
+        if (tune.lanes == 2) launch_group<MODE, false, 2, false>(s, io, num_sms, st);
+        else launch_group<MODE, false, 4, false>(s, io, num_sms, st);
+    } else if (io.ctr) {
+        launch_count<MODE, true>(s, io, tune, num_sms, st);
+    } else {
+        launch_count<MODE, false>(s, io, tune, num_sms, st);
+    }
     if (defer) {
-        if (io.ctr) launch_wide<MODE, true>(s, io, tune, num_sms, st);
-        else launch_wide<MODE, false>(s, io, tune, num_sms, st);
+        if (io.ctr) launch_deferred<MODE, true>(s, io, tune, num_sms, st);
+        else launch_deferred<MODE, false>(s, io, tune, num_sms, st);
     }
     if (io.huge) {
         if (io.ctr) launch_huge<MODE, true>(s, io, num_sms, st);

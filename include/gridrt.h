@@ -473,8 +473,8 @@ rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, const rtg_req
  *   RTG_TUNE_CELL_RECORDS 1: builds also store the triangle records in cell-list order
  *                        (48 B per reference) so traces skip the id indirection; from the next build
  *   RTG_TUNE_HEAVY_CELL  n > 0: a ray that meets a cell list longer than n is finished by a
- *                        second pass that traces it with a group of lanes (the list split
- *                        over them); default 32, 0 off.  Results are identical either way.
+ *                        second pass that traces it with a group of lanes (each at another of
+ *                        its next cells, the lists found dealt out over them); default 32, 0 off.  Results are identical either way.
  *                        A ray that then meets a list above 2,048 entries (a dense cluster)
  *                        is finished by a third pass, one block of threads per ray, when the
  *                        scene's last checked build had such a list.
@@ -490,10 +490,11 @@ rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, const rtg_req
  *                        (every block size keeps 64 registers a thread and 32 warps an SM)
  *   RTG_TUNE_LANES       lanes that trace each ray from its start: 1 (default: one ray a lane,
  *                        the long lists handed on as above), 2 or 4 (every ray walked by a group
- *                        of lanes that splits each cell's list).  Groups pay on launches too
- *                        small to fill the GPU with one ray a lane (65,536 triangles, 512^2
- *                        camera rays + their shadow rays: +41% at 2) and cost on full ones
- *                        (1024^2 frames: -44% at 2) */
+ *                        of lanes, each at another of its next cells; lists above heavy-cell x
+ *                        lanes / 2 handed on).  Groups pay on launches too small to fill the GPU
+ *                        with one ray a lane (65,536 triangles, 512^2 camera rays + their shadow
+ *                        rays, build included: 0.47 -> 0.32 ms at 2, 0.25 ms at 4) and cost on
+ *                        full ones (1024^2 frames: 0.38 -> 0.55 ms) */
 enum {
     RTG_TUNE_EMPTY_RUN = 1,
     RTG_TUNE_PERSISTENT = 2,
