@@ -228,6 +228,7 @@ TraceSlot scene_counter(rtg_scene s) {
     t.ctr = s->d_ray_ctr + 8 * (size_t)slot;
     t.defer = s->d_defer ? s->d_defer + (size_t)slot * kDeferCap : nullptr;
     t.defer_cap = s->d_defer ? kDeferCap : 0;
+    t.longest = s->hp.max_list < 0x7fffffffu ? (int32_t)s->hp.max_list : 0x7fffffff;
     // the block-per-ray pass is launched for scenes whose last checked build
     // had a list above kHugeList (the group pass handles such lists anyway)
     if (s->d_defer && s->hp.max_list > (uint32_t)kHugeList) {

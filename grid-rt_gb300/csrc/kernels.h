@@ -108,13 +108,33 @@ struct TraceTuning {
     int refill = -1;       // > 0: idle lanes take new rays once this many are idle (0: finish each batch of 32);
                            // -1 (default): 16 for rays given as arrays, off for camera and frame traces
     int block = 128;       // threads per block of the one-lane trace launch: 64, 128 or 256
-    int lanes = 1;         // lanes per ray from the start: 1 (one-lane walk), 2 or 4 (group walk)
+    int lanes = 0;         // lanes per ray from the start: 1 (one-lane walk), 2 or 4 (group walk);
+                           // 0 (default): by the launch's size (lanes_for)
 };
 // The refill threshold of a launch over camera-generated rays (camera and
 // frame traces: coherent, and in a frame each lane's shadow ray follows its
 // camera ray, which refill would interleave) or over rays given as arrays.
 inline int refill_for(const TraceTuning& t, int mode_is_camera) {
     return t.refill >= 0 ? t.refill : (mode_is_camera ? 0 : 16);
+}
+
+// Lanes per ray from the start for a launch of n rays on `sms` SMs.  A ray is a
+// chain of dependent loads, so a launch that does not fill the SMs' 1,024
+// resident lanes several times over lasts as long as its longest rays: it
+// gives each ray a group of lanes.  More lanes shorten the chain and cost
+// throughput, so the group shrinks as the launch grows.  Measured on 152 SMs
+// (155,648 lanes), us a launch at 1 / 8 / 16 / 32 lanes, random closest-hit
+// rays in 100,000 triangles: 1,000 rays 160 / 42 / 28 / 23, 16,000 rays
+// 188 / 66 / 46 / 46, 64,000 rays 231 / 126 / 102 / 120, 128,000 rays
+// 252 / 188 / 169 / 222, 256,000 rays 336 / 356 / 333 / 427; frames (each ray
+// followed by its shadow ray, uneven over the image) of the same triangles:
+// 64,000 pixels 348 / 96 / 83 / 103, 256,000 376 / 189 / 231 / 357, 512,000
+// 423 / 327 / 438 / 702 -- but 512,000 pixels of the sphere 246 / 331.
+inline int lanes_for(long long n, int sms, int mode_is_camera) {
+    const long long resident = 1024LL * sms;
+    if (8 * n <= resident) return 32;
+    if (2 * n <= resident) return 16;
+    return n <= (mode_is_camera ? 2 * resident : resident + resident / 4) ? 8 : 1;
 }
 
 // Kernel launch with programmatic stream serialisation when GRIDRT_PDL is on
@@ -147,6 +167,7 @@ struct TraceSlot {
     int32_t defer_cap;
     int2* huge = nullptr; // {ray, cell} entries of rays at a list above kHugeList (nullptr: no block pass)
     int32_t huge_cap = 0;
+    int32_t longest = 0x7fffffff;   // longest list of the scene's last checked build (unknown: the largest value)
 };
 // Lists longer than this are tested by a whole block (the block-per-ray pass)
 // when the trace's slot has a huge-list queue.

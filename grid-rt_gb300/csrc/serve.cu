@@ -124,6 +124,7 @@ extern "C" rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, co
         return RTG_DEVICE_ERROR;
     }
     TraceTuning tune = scenes[0]->tune;
+    tune.lanes = 1;   // steps of any size keep the one-lane walk: requests gather in shared steps while one runs
     if (opt->empty_run == 2 || opt->empty_run == 4 || opt->empty_run == 8 || opt->empty_run == 16)
         tune.empty_run = opt->empty_run;
 

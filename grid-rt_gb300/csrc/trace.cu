@@ -169,12 +169,13 @@ __global__ void __launch_bounds__(128, GRIDRT_TRACE_MIN_BLOCKS)
     }
 }
 
-// Group pass over the rays a batch launch deferred (flattened indices); each
-// group resolves its own task, scene and mode.
-template <int G>
+// Group walk over a batch's rays (flattened indices): those its launch deferred
+// (QUEUE), or all of a small batch's from their start; each group resolves its
+// own task, scene and mode.
+template <int G, bool QUEUE>
 __global__ void __launch_bounds__(128, GRIDRT_GROUP_BATCH_MIN_BLOCKS)
     trace_group_batch_kernel(const BatchScene* __restrict__ scenes, int nscenes, const BatchTask* __restrict__ tasks,
-                             int ntasks, unsigned long long* counter, const int2* __restrict__ defer,
+                             int ntasks, long long rays, unsigned long long* counter, const int2* __restrict__ defer,
                              int32_t defer_cap) {
     pdl_begin();
     __shared__ SParams P[kMaxBatchScenes];
@@ -182,8 +183,11 @@ __global__ void __launch_bounds__(128, GRIDRT_GROUP_BATCH_MIN_BLOCKS)
     __syncthreads();
     const int gl = threadIdx.x & (G - 1);
     constexpr int kWant = G < 32 ? 16 / G : 1;
-    unsigned long long total = counter[1];
-    if (total > (unsigned long long)defer_cap) total = (unsigned long long)defer_cap;
+    unsigned long long total = (unsigned long long)rays;
+    if (QUEUE) {
+        total = counter[1];
+        if (total > (unsigned long long)defer_cap) total = (unsigned long long)defer_cap;
+    }
     bool busy = false, exhausted = false, any = false;
     int todo = 0, scene = 0;
     int3 sg = make_int3(0, 0, 0);
@@ -192,9 +196,9 @@ __global__ void __launch_bounds__(128, GRIDRT_GROUP_BATCH_MIN_BLOCKS)
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !busy);
         if (!exhausted && __popc(idle) >= kWant * G) {
-            const unsigned long long r = claim_groups<G>(idle, counter + 2, total, exhausted);
+            const unsigned long long r = claim_groups<G>(idle, counter + (QUEUE ? 2 : 0), total, exhausted);
             if (!busy && r < total) {
-                const int2 d = __ldg(defer + r);
+                const int2 d = QUEUE ? __ldg(defer + r) : make_int2((int32_t)r, -1);
                 const BatchTask T = tasks[find_task(tasks, ntasks, (long long)d.x)];
                 scene = T.scene;
                 any = T.mode == MODE_ANY;
@@ -202,10 +206,11 @@ __global__ void __launch_bounds__(128, GRIDRT_GROUP_BATCH_MIN_BLOCKS)
                 io.occ = static_cast<uint8_t*>(T.out);
                 io.hits = static_cast<int4*>(T.out);
                 L.ray = (int32_t)((long long)d.x - T.first);
-                busy = any ? start_ray<MODE_ANY>(P[scene], io, L, L.ray) : start_ray<MODE_NEAREST>(P[scene], io, L, L.ray);
+                const bool pad = !QUEUE && L.ray >= T.n;   // a task's rays are padded to a multiple of 32
+                if (!pad) busy = any ? start_ray<MODE_ANY>(P[scene], io, L, L.ray) : start_ray<MODE_NEAREST>(P[scene], io, L, L.ray);
                 if (busy) {
-                    resume_at(P[scene], L, d.y);
-                } else {
+                    if (QUEUE) resume_at(P[scene], L, d.y);
+                } else if (!pad) {
                     if (L.id != -2) L.id = -1;
                     if (any) finish_ray<MODE_ANY>(io, P[scene], scenes[scene].view, L, gl == 0);
                     else finish_ray<MODE_NEAREST>(io, P[scene], scenes[scene].view, L, gl == 0);
@@ -451,23 +456,35 @@ static void launch_batch_er(const BatchScene* scenes, int nscenes, const BatchTa
                  slot.ctr, heavy > 0 ? slot.defer : nullptr, slot.defer_cap, heavy, refill);
 }
 
-template <int G>
+template <int G, bool QUEUE>
 static void launch_group_batch(const BatchScene* scenes, int nscenes, const BatchTask* tasks, int ntasks,
-                               const TraceSlot& slot, int num_sms, cudaStream_t st) {
+                               long long total, const TraceSlot& slot, int num_sms, cudaStream_t st) {
     static int per_sm = 0;
     if (per_sm == 0) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_group_batch_kernel<G>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_group_batch_kernel<G, QUEUE>, 128, 0);
         per_sm = b > 0 ? b : 1;
     }
-    launch_k(trace_group_batch_kernel<G>, (unsigned)(per_sm * num_sms), 128, 0, st, scenes, nscenes, tasks, ntasks,
-             slot.ctr, slot.defer, slot.defer_cap);
+    const long long full = (long long)per_sm * num_sms, need = (total + 128 / G - 1) / (128 / G);
+    launch_k(trace_group_batch_kernel<G, QUEUE>, (unsigned)(need < full ? need : full), 128, 0, st, scenes, nscenes,
+             tasks, ntasks, total, slot.ctr, slot.defer, slot.defer_cap);
 }
 
 void launch_trace_batch(const BatchScene* scenes, int nscenes, const BatchTask* tasks, int ntasks, long long total,
                         const TraceSlot& slot, const TraceTuning& tune, int num_sms, cudaStream_t st) {
     if (total <= 0 || ntasks <= 0) return;
     // deferred entries are int32 flattened indices
+    const int lanes = tune.lanes || total > 0x7fffffffLL ? 1 : lanes_for(total, num_sms, 0);
+    if (lanes > 1) {
+        // a small batch: every ray by a group of lanes, long lists dealt out
+        // over it
+        count_launches(1);
+        cudaMemsetAsync(slot.ctr, 0, 3 * sizeof(unsigned long long), st);
+        if (lanes == 32) launch_group_batch<32, false>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
+        else if (lanes == 16) launch_group_batch<16, false>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
+        else launch_group_batch<8, false>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
+        return;
+    }
     const bool defer = tune.heavy_cell > 0 && slot.defer && slot.defer_cap > 0 && total <= 0x7fffffffLL;
     const int32_t heavy = defer ? tune.heavy_cell : 0;
     count_launches(defer ? 2 : 1);
@@ -477,10 +494,10 @@ void launch_trace_batch(const BatchScene* scenes, int nscenes, const BatchTask* 
     else if (tune.empty_run <= 8) launch_batch_er<8>(scenes, nscenes, tasks, ntasks, total, slot, heavy, refill_for(tune, 0), num_sms, st);
     else launch_batch_er<16>(scenes, nscenes, tasks, ntasks, total, slot, heavy, refill_for(tune, 0), num_sms, st);
     if (defer) {
-        if (tune.heavy_lanes <= 4) launch_group_batch<4>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
-        else if (tune.heavy_lanes <= 8) launch_group_batch<8>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
-        else if (tune.heavy_lanes <= 16) launch_group_batch<16>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
-        else launch_group_batch<32>(scenes, nscenes, tasks, ntasks, slot, num_sms, st);
+        if (tune.heavy_lanes <= 4) launch_group_batch<4, true>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
+        else if (tune.heavy_lanes <= 8) launch_group_batch<8, true>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
+        else if (tune.heavy_lanes <= 16) launch_group_batch<16, true>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
+        else launch_group_batch<32, true>(scenes, nscenes, tasks, ntasks, total, slot, num_sms, st);
     }
 }
 

@@ -822,7 +822,8 @@ __device__ __forceinline__ void resume_at(const SParams& P, Lane& L, int32_t cel
 // ---------------------------------------------------------------------------
 // Group walk: G lanes trace one ray together, lane j at the j-th next cell of
 // its walk.  Used for the rays the one-lane walk defers (a long list, or many
-// tests made already) and for every ray of a launch with RTG_TUNE_LANES 2 or 4.
+// tests made already) and for every ray of a small launch (lanes_for) or of one
+// with RTG_TUNE_LANES 2 or 4.
 //
 // Bound by latency: a walk is a chain of dependent loads (occupancy word, list
 // bounds, ids, records) of ~1 us a non-empty cell, and a launch ends with its
@@ -1462,23 +1463,35 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
     io.defer = defer ? slot.defer : nullptr;
     io.defer_cap = defer ? slot.defer_cap : 0;
     io.heavy = defer ? tune.heavy_cell : kNoHeavy;
-    io.refill = refill_for(tune, MODE == MODE_CAMERA || MODE == MODE_FRAME);
+    constexpr int camera = MODE == MODE_CAMERA || MODE == MODE_FRAME;
+    io.refill = refill_for(tune, camera);
     io.huge = defer ? slot.huge : nullptr;
     io.huge_cap = io.huge ? slot.huge_cap : 0;
     cudaMemsetAsync(slot.ctr, 0, 8 * sizeof(unsigned long long), st);
-    count_launches(defer ? (io.huge ? 3 : 2) : 1);
-    if (tune.lanes > 1 && !io.ctr) {
-        // every ray walked by a group of lanes from its start; a list that
-        // would take its lanes more than heavy_cell / 2 turns is deferred
-        if (defer && io.heavy < kNoHeavy / 4) io.heavy = io.heavy * tune.lanes / 2;
-        if (tune.lanes == 2) launch_group<MODE, false, 2, false>(s, io, num_sms, st);
-        else launch_group<MODE, false, 4, false>(s, io, num_sms, st);
-    } else if (io.ctr) {
-        launch_count<MODE, true>(s, io, tune, num_sms, st);
-    } else {
-        launch_count<MODE, false>(s, io, tune, num_sms, st);
+    const int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera));
+    if (lanes > 1) {
+        // every ray walked by a group of lanes from its start.  A list that
+        // would take its lanes more than heavy_cell / 2 turns is deferred;
+        // groups of 16 and 32 deal any list out themselves, as do all when
+        // the scene had no such list
+        if (io.heavy < kNoHeavy / 64) io.heavy = io.heavy * lanes / 2;
+        if (lanes >= 16 || (!tune.lanes && slot.longest <= io.heavy)) {
+            io.defer = nullptr;
+            io.defer_cap = 0;
+        }
     }
-    if (defer) {
+    count_launches(1 + (io.defer ? 1 : 0) + (io.huge ? 1 : 0));
+    switch (lanes) {
+        case 2: launch_group<MODE, false, 2, false>(s, io, num_sms, st); break;
+        case 4: launch_group<MODE, false, 4, false>(s, io, num_sms, st); break;
+        case 8: launch_group<MODE, false, 8, false>(s, io, num_sms, st); break;
+        case 16: launch_group<MODE, false, 16, false>(s, io, num_sms, st); break;
+        case 32: launch_group<MODE, false, 32, false>(s, io, num_sms, st); break;
+        default:
+            if (io.ctr) launch_count<MODE, true>(s, io, tune, num_sms, st);
+            else launch_count<MODE, false>(s, io, tune, num_sms, st);
+    }
+    if (io.defer) {
         if (io.ctr) launch_deferred<MODE, true>(s, io, tune, num_sms, st);
         else launch_deferred<MODE, false>(s, io, tune, num_sms, st);
     }

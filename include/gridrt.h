@@ -488,13 +488,14 @@ rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, const rtg_req
  *                        and frame traces, whose lanes follow a camera ray with its shadow ray
  *   RTG_TUNE_BLOCK       threads per block of the one-lane trace launch: 64, 128 (default) or 256
  *                        (every block size keeps 64 registers a thread and 32 warps an SM)
- *   RTG_TUNE_LANES       lanes that trace each ray from its start: 1 (default: one ray a lane,
- *                        the long lists handed on as above), 2 or 4 (every ray walked by a group
- *                        of lanes, each at another of its next cells; lists above heavy-cell x
- *                        lanes / 2 handed on).  Groups pay on launches too small to fill the GPU
- *                        with one ray a lane (65,536 triangles, 512^2 camera rays + their shadow
- *                        rays, build included: 0.47 -> 0.32 ms at 2, 0.25 ms at 4) and cost on
- *                        full ones (1024^2 frames: 0.38 -> 0.55 ms) */
+ *   RTG_TUNE_LANES       lanes that trace each ray from its start: 1 (one ray a lane, the long
+ *                        lists handed on as above), 2 or 4 (every ray walked by a group of lanes,
+ *                        each at another of its next cells; lists above heavy-cell x lanes / 2
+ *                        handed on).  Unset, launches too small to fill the GPU with one ray a
+ *                        lane use groups of 32, 16 or 8 lanes by their size and larger ones one
+ *                        lane (65,536 triangles, 512^2 camera rays + their shadow rays, build
+ *                        included: 0.47 ms at 1 lane, 0.32 at 2, 0.24 unset; 1024^2 frames:
+ *                        0.38 ms at 1, 0.55 at 2 or 4) */
 enum {
     RTG_TUNE_EMPTY_RUN = 1,
     RTG_TUNE_PERSISTENT = 2,
