@@ -106,7 +106,7 @@ struct TraceTuning {
     int heavy_cell = 32;   // > 0: rays meeting a list longer than this finish in a warp-per-ray pass
     int heavy_lanes = 32;  // lanes per deferred ray in that pass: 4, 8, 16 or 32
     int refill = -1;       // > 0: idle lanes take new rays once this many are idle (0: finish each batch of 32);
-                           // -1 (default): 16 for rays given as arrays, off for camera and frame traces
+                           // -1 (default): 8 for rays given as arrays, off for camera and frame traces
     int block = 128;       // threads per block of the one-lane trace launch: 64, 128 or 256
     int lanes = 0;         // lanes per ray from the start: 1 (one-lane walk), 2 or 4 (group walk);
                            // 0 (default): by the launch's size (lanes_for)
@@ -115,7 +115,7 @@ struct TraceTuning {
 // frame traces: coherent, and in a frame each lane's shadow ray follows its
 // camera ray, which refill would interleave) or over rays given as arrays.
 inline int refill_for(const TraceTuning& t, int mode_is_camera) {
-    return t.refill >= 0 ? t.refill : (mode_is_camera ? 0 : 16);
+    return t.refill >= 0 ? t.refill : (mode_is_camera ? 0 : 8);
 }
 
 // Lanes per ray from the start for a launch of n rays on `sms` SMs.  A ray is a

@@ -21,81 +21,76 @@ __device__ __forceinline__ int find_task(const BatchTask* __restrict__ tasks, in
     return lo;
 }
 
-// Lane refill inside one batch task (TraceIO::refill > 0): the warp draws
-// 32-ray chunks from the flattened counter and hands their rays to idle
-// lanes while the chunks belong to its task, so scene and mode stay
-// warp-uniform; a chunk of a later task ends the task here once its rays
-// are finished and is returned (or a value >= total at the end).
-template <int MODE, int ER>
+// Lane refill inside one batch task: the warp draws 32-ray chunks from the
+// flattened counter and hands their rays to idle lanes while the chunks belong
+// to its task, so scene and mode stay warp-uniform; starts on the task's chunk
+// at `base`, and returns the first chunk past the task once its rays are
+// finished.
+template <int ER>
 __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P, const SceneView& s,
-                                                                const TraceIO& io, Lane& L, long long tfirst,
-                                                                unsigned long long chunk, long long total,
-                                                                uint32_t& cells, uint32_t& tests,
+                                                                const TraceIO& io, Lane& L, long long first,
+                                                                int32_t base, uint32_t& cells, uint32_t& tests,
                                                                 uint32_t& started) {
     const int lane = threadIdx.x & 31;
-    long long pb = (long long)chunk - tfirst;                 // task-local rays not yet started: [pb, pe)
-    long long pe = pb + 32 < io.n ? pb + 32 : io.n;
-    unsigned long long next = ~0ull;                          // a claimed chunk past this task
+    const int32_t n = (int32_t)io.n;
+    int32_t at = base, left = min(32, n - base);   // the chunk's next ray, and how many it still has
+    unsigned long long next = ~0ull;               // a claimed chunk past this task
     bool active = false;
-    int32_t heavy = io.heavy, work_cap = kNoHeavy;
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !active);
         const int nidle = __popc(idle);
         const bool room = nidle >= io.refill || idle == FULL;
-        if (pb >= pe && next == ~0ull && room) {
-            unsigned long long nb = 0;
-            if (lane == 0) nb = atomicAdd(io.counter, 32ull);
-            nb = __shfl_sync(FULL, nb, 0);
-            if ((long long)nb < tfirst + io.n) {
-                pb = (long long)nb - tfirst;
-                pe = pb + 32 < io.n ? pb + 32 : io.n;
+        if (left == 0 && next == ~0ull && room) {
+            unsigned long long b = 0;
+            if (lane == 0) b = atomicAdd(io.counter, 32ull);
+            b = __shfl_sync(FULL, b, 0);
+            if ((long long)b - first < (long long)n) {
+                at = (int32_t)((long long)b - first);
+                left = min(32, n - at);
             } else {
-                next = nb;
+                next = b;
             }
         }
-        if (pb < pe && room) {
-            const int take = (long long)nidle < pe - pb ? nidle : (int)(pe - pb);
+        if (left > 0 && room) {
+            const int take = min(nidle, left);
             if (!active) {
                 const int rank = __popc(idle & ((1u << lane) - 1u));
                 if (rank < take) {
-                    L.ray = (int32_t)(pb + rank);
-                    heavy = io.heavy;
-                    work_cap = heavy < kNoHeavy / (kHeavyWorkMult + 1) && kHeavyWorkMult > 0 ? heavy * kHeavyWorkMult
-                                                                                             : kNoHeavy;
+                    L.ray = at + rank;
+                    set_deferral(L, io.heavy);
                     ++started;
-                    if (start_ray<MODE>(P, io, L, L.ray)) {
+                    if (start_ray<MODE_TASK>(P, io, L, L.ray)) {
                         active = true;
                     } else {
                         if (L.id != -2) L.id = -1;
-                        finish_ray<MODE>(io, P, s, L);
+                        finish_ray<MODE_TASK>(io, P, s, L);
                     }
                 }
             }
-            pb += take;
+            at += take;
+            left -= take;
         }
         if (!__any_sync(FULL, active)) {
-            if (pb >= pe && next != ~0ull) return next;
+            if (left == 0 && next != ~0ull) return next;
             continue;
         }
-        bool fin = active &&
-                   advance<MODE, ER>(P, L, s.offsets, s.ids, s.tris, s.wald, s.occ, s.crec, heavy, work_cap, cells, tests);
+        bool fin = advance_two<MODE_TASK, ER>(P, L, s, active, cells, tests);
         if (io.defer) {
             const bool d = fin && L.id == kDeferred;
             const unsigned m = __ballot_sync(FULL, d);
             if (m) {
                 const int leader = __ffs(m) - 1;
-                unsigned long long at = 0;
-                if (lane == leader) at = atomicAdd(io.counter + 1, (unsigned long long)__popc(m));
-                at = __shfl_sync(FULL, at, leader);
+                unsigned long long slot0 = 0;
+                if (lane == leader) slot0 = atomicAdd(io.counter + 1, (unsigned long long)__popc(m));
+                slot0 = __shfl_sync(FULL, slot0, leader);
                 if (d) {
-                    const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
+                    const unsigned long long slot = slot0 + __popc(m & ((1u << lane) - 1u));
                     if (slot < (unsigned long long)io.defer_cap) {
-                        io.defer[slot] = make_int2(defer_tag<MODE>(L, io),
+                        io.defer[slot] = make_int2(defer_tag<MODE_TASK>(L, io),
                                                    L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
                         active = false;
                     } else {
-                        heavy = kNoHeavy;
-                        work_cap = kNoHeavy;
+                        set_deferral(L, kNoHeavy);
                         L.id = -1;
                     }
                     fin = false;
@@ -103,7 +98,7 @@ __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P
             }
         }
         if (fin) {
-            finish_ray<MODE>(io, P, s, L);
+            finish_ray<MODE_TASK>(io, P, s, L);
             active = false;
         }
     }
@@ -118,7 +113,7 @@ __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P
 // Many (scene, ray batch) tasks in one persistent launch.  Task t owns the
 // 32-aligned index range [first, first + n) of one flattened ray space, so a
 // 32-ray claim always falls inside one task: scene and mode are warp-uniform.
-template <int ER, bool REFILL>
+template <int ER>
 __global__ void __launch_bounds__(128, GRIDRT_TRACE_MIN_BLOCKS)
     trace_batch_kernel(const BatchScene* __restrict__ scenes, int nscenes, const BatchTask* __restrict__ tasks,
                        int ntasks, long long total, unsigned long long* counter, int2* defer, int32_t defer_cap,
@@ -145,27 +140,17 @@ __global__ void __launch_bounds__(128, GRIDRT_TRACE_MIN_BLOCKS)
         io.heavy = defer ? heavy : kNoHeavy;
         io.defer_base = (int32_t)T.first;
         io.refill = refill;
-        if (REFILL) {
-            if (T.mode == MODE_ANY) {
-                io.occ = static_cast<uint8_t*>(T.out);
-                b = trace_task_refill<MODE_ANY, ER>(P[T.scene], V, io, L, T.first, b, total, cells, tests, started);
-            } else {
-                io.hits = static_cast<int4*>(T.out);
-                b = trace_task_refill<MODE_NEAREST, ER>(P[T.scene], V, io, L, T.first, b, total, cells, tests,
-                                                        started);
-            }
-            continue;
-        }
-        const long long base = (long long)b - T.first;
-        if (T.mode == MODE_ANY) {
-            io.occ = static_cast<uint8_t*>(T.out);
-            trace_batch32<MODE_ANY, ER>(P[T.scene], V, io, L, base, cells, tests, started);
+        io.any = T.mode == MODE_ANY;
+        io.occ = static_cast<uint8_t*>(T.out);
+        io.hits = static_cast<int4*>(T.out);
+        const int32_t base = (int32_t)((long long)b - T.first);
+        if (refill > 0 && !chunk_coherent(P[T.scene], io, base)) {
+            b = trace_task_refill<ER>(P[T.scene], V, io, L, T.first, base, cells, tests, started);
         } else {
-            io.hits = static_cast<int4*>(T.out);
-            trace_batch32<MODE_NEAREST, ER>(P[T.scene], V, io, L, base, cells, tests, started);
+            trace_batch32<MODE_TASK, ER>(P[T.scene], V, io, L, base, cells, tests, started);
+            if (lane == 0) b = atomicAdd(counter, 32ull);
+            b = __shfl_sync(FULL, b, 0);
         }
-        if (lane == 0) b = atomicAdd(counter, 32ull);
-        b = __shfl_sync(FULL, b, 0);
     }
 }
 
@@ -327,21 +312,18 @@ __global__ void __launch_bounds__(128) trace_instances_kernel(const InstanceRec*
                 xf_dir(m, wd[0], wd[1], wd[2], L.dx, L.dy, L.dz);
                 active = setup_ray(P, L, tn, tf);
                 L.tmax = tmax;
+                set_deferral(L, kNoHeavy);
                 if (MODE == MODE_NEAREST) L.best = gbest;
             }
-            const int32_t* offs = R->view.offsets;
-            const int32_t* ids = R->view.ids;
-            const float4* tris = R->view.tris;
-            const uint32_t* occ = R->view.occ;
-            const float4* crec = R->view.crec;
+            const SceneView V = R->view;
             while (__any_sync(FULL, active)) {
-                if (active && advance<MODE, ER>(P, L, offs, ids, tris, R->view.wald, occ, crec, kNoHeavy, kNoHeavy, cells, tests)) {
+                if (advance<MODE, ER>(P, L, V, active, cells, tests)) {
                     active = false;
                     if (L.id >= 0) {
                         // the next instance compares against the exact
                         // distance (the walk may have accepted its hit on
                         // Moller-Trumbore's t)
-                        gbest = wald_f_of(L, L.id, R->view.wald);
+                        gbest = wald_f_of(L, L.id, V.wald);
                         gid = L.id;
                         ginst = i;
                         if (MODE == MODE_ANY) alive = false;   // occluded
@@ -442,18 +424,14 @@ static void launch_batch_er(const BatchScene* scenes, int nscenes, const BatchTa
     static int per_sm = 0;
     if (per_sm == 0) {
         int b = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_batch_kernel<ER, false>, 128, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, trace_batch_kernel<ER>, 128, 0);
         per_sm = b > 0 ? b : 1;
     }
     long long blocks = (total + 127) / 128;
     blocks = blocks < (long long)per_sm * num_sms ? blocks : (long long)per_sm * num_sms;
     if (blocks < 1) blocks = 1;
-    if (refill > 0)
-        launch_k(trace_batch_kernel<ER, true>, (unsigned)blocks, 128, 0, st, scenes, nscenes, tasks, ntasks, total,
-                 slot.ctr, heavy > 0 ? slot.defer : nullptr, slot.defer_cap, heavy, refill);
-    else
-        launch_k(trace_batch_kernel<ER, false>, (unsigned)blocks, 128, 0, st, scenes, nscenes, tasks, ntasks, total,
-                 slot.ctr, heavy > 0 ? slot.defer : nullptr, slot.defer_cap, heavy, refill);
+    launch_k(trace_batch_kernel<ER>, (unsigned)blocks, 128, 0, st, scenes, nscenes, tasks, ntasks, total, slot.ctr,
+             heavy > 0 ? slot.defer : nullptr, slot.defer_cap, heavy, refill);
 }
 
 template <int G, bool QUEUE>

@@ -33,6 +33,8 @@
 
 namespace gridrt {
 
+static constexpr float kChunkCells = 4.0f;   // chunk_coherent: origins, in cells
+static constexpr float kChunkCone = 0.1f;    // and directions, of the first ray's length
 static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the warp-per-ray pass
 static constexpr int32_t kNoHeavy = 0x7fffffff;
@@ -47,7 +49,9 @@ static constexpr int32_t kHeavyWorkMult = GRIDRT_HEAVY_WORK_MULT;
 // MODE_FRAME: a camera ray, then in the same lane the shadow ray of its hit
 // (any-hit); Lane::tmax is -inf in the camera phase and the shadow ray's
 // tmax after.
-enum Mode : int { MODE_NEAREST = 0, MODE_ANY = 1, MODE_CAMERA = 2, MODE_FRAME = 3 };
+// MODE_TASK: a batch task's rays, closest hits or occlusion as TraceIO::any
+// says (Lane::tmax is -inf for closest hits), one copy of the walk for both.
+enum Mode : int { MODE_NEAREST = 0, MODE_ANY = 1, MODE_CAMERA = 2, MODE_FRAME = 3, MODE_TASK = 4 };
 
 struct SParams {
     float bmin[3], bmax[3], cell[3], inv[3];
@@ -83,13 +87,29 @@ struct Lane {
     float tMx, tMy, tMz, tDx, tDy, tDz;
     int32_t x, y, z;
     int32_t budget;
-    int32_t work;        // triangle tests made so far by this ray
+    int32_t work;        // triangle tests this ray may still make before it is deferred
+    int32_t heavy;       // lists longer than this defer it
     float best;
     int32_t id;
     int32_t cw;          // cached occupancy word index
     uint32_t cword;      // its value
     int32_t ray;         // ray index within the launch or task, -1 = none
+    int32_t li, le;      // entries of the current cell's list not yet tested (advance); li >= le: walking
+    bool fast_best;      // best is Moller-Trumbore's t of an accepted entry (test_tri_fast)
 };
+
+// Whether the lane's ray looks for occlusion before L.tmax.
+template <int MODE>
+__device__ __forceinline__ bool any_hit_phase(const Lane& L) {
+    return MODE == MODE_ANY || ((MODE == MODE_FRAME || MODE == MODE_TASK) && L.tmax > -kFltMax);
+}
+
+// When the one-lane walk hands the lane's ray on: at a list above `heavy`, or
+// once its tests would pass kHeavyWorkMult x heavy (kNoHeavy: never).
+__device__ __forceinline__ void set_deferral(Lane& L, int32_t heavy) {
+    L.heavy = heavy;
+    L.work = heavy < kNoHeavy / (kHeavyWorkMult + 1) && kHeavyWorkMult > 0 ? heavy * kHeavyWorkMult : kNoHeavy;
+}
 
 // Ray::update + AabbIntersection::clipRay + traverse3ddda set-up
 // (include/rt/Ray.h:26-37, src/rtcore/AabbIntersection.cpp:37-63,
@@ -129,10 +149,10 @@ __device__ __forceinline__ bool setup_ray(const SParams& P, Lane& L, float tnear
     // A walk visits at most nx+ny+nz-2 cells; the bound only guards against a
     // zero direction component (outside the reference's domain) looping.
     L.budget = P.res[0] + P.res[1] + P.res[2] + 3;
-    L.work = 0;
     L.best = kFltMax;
     L.id = -1;
     L.cw = -1;
+    L.li = L.le = 0;
     return true;
 }
 
@@ -229,7 +249,7 @@ __device__ __forceinline__ bool wald_decide(Lane& L, int32_t tid, float hi, cons
     if (fsub(fsub(1.0f, lambda), mue) < 0.0f) return false;
     L.best = f;
     L.id = tid;
-    return (MODE == MODE_ANY || MODE == MODE_FRAME) && f < L.tmax;
+    return (MODE == MODE_ANY || MODE == MODE_FRAME || MODE == MODE_TASK) && f < L.tmax;
 }
 
 template <int MODE>
@@ -271,7 +291,7 @@ __device__ __forceinline__ bool test_tri(Lane& L, int32_t tid, const float4& A, 
     if (acc) {
         L.best = t;
         L.id = tid;
-        if ((MODE == MODE_ANY || MODE == MODE_FRAME) && t < L.tmax) return true;
+        if ((MODE == MODE_ANY || MODE == MODE_FRAME || MODE == MODE_TASK) && t < L.tmax) return true;
     }
     return false;
 #endif
@@ -323,7 +343,7 @@ __device__ __forceinline__ bool test_tri_fast(Lane& L, int32_t tid, const float4
     const float t = (C.x * qx + C.y * qy + C.z * qz) * idet;
     const float ts = fabsf(t) * kMtTRelSlack + kHitEpsilon;
     if (!((t < L.best + ts) && (t >= L.lo - ts) && (t <= hi + ts))) return false;
-    const bool any_phase = MODE == MODE_ANY || (MODE == MODE_FRAME && L.tmax > -kFltMax);
+    const bool any_phase = any_hit_phase<MODE>(L);
     if (u >= kMtBarySlack && v >= kMtBarySlack && w >= kMtBarySlack && t >= L.lo + ts && t <= hi - ts &&
         t < L.best - ts && (!any_phase || t < L.tmax - ts || t > L.tmax + ts)) {
         L.best = t;
@@ -341,26 +361,42 @@ __device__ __forceinline__ bool test_tri_fast(Lane& L, int32_t tid, const float4
 #endif
 }
 
-// Visits up to ER empty cells and at most one non-empty cell.
-// Returns true when the ray is finished (hit decided, or left the grid).
-template <int MODE, int ER>
-__device__ __forceinline__ bool advance(const SParams& P, Lane& L, const int32_t* __restrict__ offsets,
-                                        const int32_t* __restrict__ ids, const float4* __restrict__ tris,
-                                        const float4* __restrict__ wald,
-                                        const uint32_t* __restrict__ occ, const float4* __restrict__ crec,
-                                        int32_t heavy, int32_t work_cap, uint32_t& cells, uint32_t& tests) {
+// Tests list entries i and (when i + 1 < e) i + 1, both records loaded before
+// either is tested.  True when an any-hit ray is occluded.
+template <int MODE>
+__device__ __forceinline__ bool test_two(Lane& L, const SceneView& s, int32_t i, int32_t e, float hi) {
+    const int32_t i1 = min(i + 1, e - 1);
+    int32_t t0 = i, t1 = i1;
+    const float4* __restrict__ recs = s.crec;   // in cell-list order: no id indirection
+    if (!s.crec) {
+        t0 = __ldg(s.ids + i);
+        t1 = __ldg(s.ids + i1);
+        recs = s.tris;
+    }
+    const float4 A0 = __ldg(recs + 3 * (int64_t)t0), B0 = __ldg(recs + 3 * (int64_t)t0 + 1),
+                 C0 = __ldg(recs + 3 * (int64_t)t0 + 2);
+    const float4 A1 = __ldg(recs + 3 * (int64_t)t1), B1 = __ldg(recs + 3 * (int64_t)t1 + 1),
+                 C1 = __ldg(recs + 3 * (int64_t)t1 + 2);
+    if (test_tri_fast<MODE>(L, __float_as_int(A0.w), A0, B0, C0, hi, s.wald, L.fast_best)) return true;
+    return i1 > i && test_tri_fast<MODE>(L, __float_as_int(A1.w), A1, B1, C1, hi, s.wald, L.fast_best);
+}
+
+// Walks a lane past up to ER empty cells.  At a non-empty cell sets [L.li, L.le)
+// to its list.  True when the ray leaves the grid or is deferred.
+template <int ER>
+__device__ __forceinline__ bool walk(const SParams& P, Lane& L, const SceneView& s, uint32_t& cells, uint32_t& tests) {
     const int32_t nx = P.res[0], nxy = P.res[0] * P.res[1];
-    for (int s = 0; s < ER; ++s) {
+    for (int q = 0; q < ER; ++q) {
         ++cells;
         const int32_t w = (L.x >> 2) + (L.y >> 2) * P.bx + (L.z >> 1) * P.bxby;
         if (w != L.cw) {
             L.cw = w;
-            L.cword = __ldg(occ + w);
+            L.cword = __ldg(s.occ + w);
         }
         if (L.cword & occ_bit(L.x, L.y, L.z)) {
             const int32_t c = L.x + L.y * nx + L.z * nxy;
-            const int32_t b = __ldg(offsets + c), e = __ldg(offsets + c + 1);
-            if (e - b > heavy || L.work > work_cap - (e - b)) {
+            const int32_t b = __ldg(s.offsets + c), e = __ldg(s.offsets + c + 1);
+            if (e - b > min(L.heavy, L.work)) {
                 // a long list, or a ray that has made many tests already
                 // (grazing a surface): the ray goes to the deferred pass,
                 // which resumes the walk at this cell (and counts it)
@@ -368,55 +404,11 @@ __device__ __forceinline__ bool advance(const SParams& P, Lane& L, const int32_t
                 L.id = kDeferred;
                 return true;
             }
-            L.work += e - b;
-            const float hi = fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon);
+            L.work -= e - b;
             tests += (uint32_t)(e - b);
-            bool fast_best = false;
-            int32_t i = b;
-            if (crec) {
-                // records stored in cell-list order: no id indirection
-                for (; i + 1 < e; i += 2) {
-                    const float4 A0 = __ldg(crec + 3 * (int64_t)i), B0 = __ldg(crec + 3 * (int64_t)i + 1),
-                                 C0 = __ldg(crec + 3 * (int64_t)i + 2);
-                    const float4 A1 = __ldg(crec + 3 * (int64_t)i + 3), B1 = __ldg(crec + 3 * (int64_t)i + 4),
-                                 C1 = __ldg(crec + 3 * (int64_t)i + 5);
-                    if (test_tri_fast<MODE>(L, __float_as_int(A0.w), A0, B0, C0, hi, wald, fast_best)) return true;
-                    if (test_tri_fast<MODE>(L, __float_as_int(A1.w), A1, B1, C1, hi, wald, fast_best)) return true;
-                }
-                if (i < e) {
-                    const float4 A0 = __ldg(crec + 3 * (int64_t)i), B0 = __ldg(crec + 3 * (int64_t)i + 1),
-                                 C0 = __ldg(crec + 3 * (int64_t)i + 2);
-                    if (test_tri_fast<MODE>(L, __float_as_int(A0.w), A0, B0, C0, hi, wald, fast_best)) return true;
-                }
-                i = e;
-            }
-            for (; i + 1 < e; i += 2) {
-                const int32_t t0 = __ldg(ids + i), t1 = __ldg(ids + i + 1);
-                const float4 A0 = __ldg(tris + 3 * (int64_t)t0), B0 = __ldg(tris + 3 * (int64_t)t0 + 1),
-                             C0 = __ldg(tris + 3 * (int64_t)t0 + 2);
-                const float4 A1 = __ldg(tris + 3 * (int64_t)t1), B1 = __ldg(tris + 3 * (int64_t)t1 + 1),
-                             C1 = __ldg(tris + 3 * (int64_t)t1 + 2);
-                if (test_tri_fast<MODE>(L, t0, A0, B0, C0, hi, wald, fast_best)) return true;
-                if (test_tri_fast<MODE>(L, t1, A1, B1, C1, hi, wald, fast_best)) return true;
-            }
-            if (i < e) {
-                const int32_t t0 = __ldg(ids + i);
-                const float4 A0 = __ldg(tris + 3 * (int64_t)t0), B0 = __ldg(tris + 3 * (int64_t)t0 + 1),
-                             C0 = __ldg(tris + 3 * (int64_t)t0 + 2);
-                if (test_tri_fast<MODE>(L, t0, A0, B0, C0, hi, wald, fast_best)) return true;
-            }
-            if (L.id >= 0) {
-                // a hit closer than the best on entry (the one-geometry walk
-                // starts from FLT_MAX; an instance walk from the instances
-                // before it).  Any-hit: the first cell with a hit decides --
-                // here not before tmax
-                if (MODE == MODE_ANY || (MODE == MODE_FRAME && L.tmax > -kFltMax)) L.id = -1;
-                return true;
-            }
-            if (dda_step(P, L)) {
-                L.id = -1;
-                return true;
-            }
+            L.fast_best = false;
+            L.li = b;
+            L.le = e;
             return false;
         }
         if (dda_step(P, L)) {
@@ -425,6 +417,64 @@ __device__ __forceinline__ bool advance(const SParams& P, Lane& L, const int32_t
         }
     }
     return false;
+}
+
+// The end of a cell's list: a hit closer than the best on entry (the
+// one-geometry walk starts from FLT_MAX; an instance walk from the instances
+// before it) ends the ray -- any-hit: the first cell with a hit decides, here
+// not before tmax -- else the ray steps on.  True when the ray is finished.
+template <int MODE>
+__device__ __forceinline__ bool leave_cell(const SParams& P, Lane& L) {
+    if (L.id >= 0) {
+        if (any_hit_phase<MODE>(L)) L.id = -1;
+        return true;
+    }
+    if (dda_step(P, L)) {
+        L.id = -1;
+        return true;
+    }
+    return false;
+}
+
+// One turn of a warp's lanes, each finishing the list it comes to (coherent
+// rays: the lanes of a warp meet the same lists).  True for a lane whose ray is
+// finished (hit decided, left the grid, or deferred).
+template <int MODE, int ER>
+__device__ __forceinline__ bool advance(const SParams& P, Lane& L, const SceneView& s, bool active, uint32_t& cells,
+                                        uint32_t& tests) {
+    bool fin = false;
+    if (active) {
+        L.li = L.le = 0;
+        fin = walk<ER>(P, L, s, cells, tests);
+    }
+    if (active && !fin && L.li < L.le) {
+        const float hi = fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon);
+        for (; L.li < L.le && !fin; L.li += 2) fin = test_two<MODE>(L, s, L.li, L.le, hi);
+        if (!fin) fin = leave_cell<MODE>(P, L);
+    }
+    return fin;
+}
+
+// One turn of a warp's lanes among incoherent rays: lanes between lists walk,
+// lanes at a list test two of its entries, so a long list does not hold up the
+// warp's other rays.  Whole lists a turn left 7.7 of 32 lanes active on random
+// rays; with this turn and refill at 8 idle lanes instead of 16, 4 M closest-hit
+// rays went from 2,468 to 2,237 us, 700,001 occlusion segments from 749 to
+// 576 us.  Coherent rays do better by whole lists (1024^2 camera rays of the
+// sphere given as an array: 246 us, by two entries a turn 349 us).
+template <int MODE, int ER>
+__device__ __forceinline__ bool advance_two(const SParams& P, Lane& L, const SceneView& s, bool active,
+                                            uint32_t& cells, uint32_t& tests) {
+    bool fin = false;
+    // half the empty cells of a coherent turn: lanes at a list wait for them
+    if (active && L.li >= L.le) fin = walk<(ER > 2 ? ER / 2 : ER)>(P, L, s, cells, tests);
+    if (active && !fin && L.li < L.le) {
+        const float hi = fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon);
+        fin = test_two<MODE>(L, s, L.li, L.le, hi);
+        L.li += 2;
+        if (!fin && L.li >= L.le) fin = leave_cell<MODE>(P, L);
+    }
+    return fin;
 }
 
 // Reported hit values of the winning triangle: RayTriIntersection::hitWald
@@ -491,6 +541,7 @@ struct TraceIO {
     int32_t heavy;                 // lists longer than this are deferred (kNoHeavy: never)
     int32_t defer_base;            // added to a deferred ray's index (a batch task's first)
     int32_t refill;                // > 0: lane refill at this many idle lanes (trace_refill)
+    int any;                       // TASK: occlusion (else closest hits)
     int2* huge;                    // rays at a list above kHugeList, for the block pass (nullptr: none)
     int32_t huge_cap;
 };
@@ -518,7 +569,7 @@ __device__ __forceinline__ bool start_ray(const SParams& P, const TraceIO& io, L
         L.dx = b.x; L.dy = b.y; L.dz = b.z;
         tnear = a.w;
         tfar = b.w;
-        if (MODE == MODE_ANY && tfar < 0.0f) {   // no shadow ray for this slot
+        if ((MODE == MODE_ANY || (MODE == MODE_TASK && io.any)) && tfar < 0.0f) {   // no shadow ray for this slot
             L.id = -2;
             return false;
         }
@@ -527,7 +578,7 @@ __device__ __forceinline__ bool start_ray(const SParams& P, const TraceIO& io, L
     L.best = kFltMax;
     if (P.failed) return false;
     const bool ok = setup_ray(P, L, tnear, tfar);
-    if (MODE == MODE_FRAME) L.tmax = -INFINITY;
+    if (MODE == MODE_FRAME || (MODE == MODE_TASK && !io.any)) L.tmax = -INFINITY;
     return ok;
 }
 
@@ -567,7 +618,7 @@ __device__ __forceinline__ bool finish_ray(const TraceIO& io, const SParams& P, 
     const float4* __restrict__ tris = sv.tris;
     const float4* __restrict__ wald = sv.wald;
     const int64_t r = L.ray;
-    if (MODE == MODE_ANY || (MODE == MODE_FRAME && L.tmax > -kFltMax)) {
+    if (MODE == MODE_TASK ? io.any != 0 : any_hit_phase<MODE>(L)) {
         if (write) io.occ[r] = L.id == -2 ? 2 : (L.id >= 0 ? 1 : 0);
         return false;
     }
@@ -648,9 +699,7 @@ __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView&
     const long long ray = base + lane;
     bool active = ray < io.n;
     L.ray = (int32_t)ray;
-    int32_t heavy = io.heavy;
-    int32_t work_cap = heavy < kNoHeavy / (kHeavyWorkMult + 1) && kHeavyWorkMult > 0 ? heavy * kHeavyWorkMult
-                                                                                    : kNoHeavy;
+    set_deferral(L, io.heavy);
     if (active) {
         ++started;
         if (!start_ray<MODE>(P, io, L, L.ray)) {
@@ -659,8 +708,7 @@ __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView&
         }
     }
     while (__any_sync(FULL, active)) {
-        bool fin = active &&
-                   advance<MODE, ER>(P, L, s.offsets, s.ids, s.tris, s.wald, s.occ, s.crec, heavy, work_cap, cells, tests);
+        bool fin = advance<MODE, ER>(P, L, s, active, cells, tests);
         if (io.defer) {
             // warp-aggregated push of the lanes that met a long list
             const bool d = fin && L.id == kDeferred;
@@ -677,8 +725,7 @@ __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView&
                         io.defer[slot] = make_int2(defer_tag<MODE>(L, io), L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
                         active = false;
                     } else {
-                        heavy = kNoHeavy;        // queue full: the lane tests the cell itself
-                        work_cap = kNoHeavy;
+                        set_deferral(L, kNoHeavy);   // queue full: the lane tests the cell itself
                         L.id = -1;
                     }
                     fin = false;
@@ -703,39 +750,69 @@ __device__ __forceinline__ void flush_counters(TraceCounters* ctr, uint32_t star
     }
 }
 
-// Eight blocks of 128 threads per SM (64 registers a thread): the walk is
-// latency-bound, and resident warps matter more than the few spilled words.
+// Eight blocks of 128 threads per SM (64 registers a thread) for camera rays:
+// the walk is latency-bound, and resident warps matter more than the few
+// spilled words.  Seven for rays given as arrays, whose kernel holds both the
+// coherent and the refilled walk: 4 M random closest-hit rays take 2,288 us at
+// seven, 2,425 at eight, 2,395 at six.
 #ifndef GRIDRT_TRACE_MIN_BLOCKS
 #define GRIDRT_TRACE_MIN_BLOCKS 8
 #endif
+constexpr int trace_min_blocks(int mode, int tpb) {
+    return (mode == MODE_NEAREST || mode == MODE_ANY) && tpb <= 128 ? 7 * 128 / tpb : GRIDRT_TRACE_MIN_BLOCKS * 128 / tpb;
+}
 
-// Lane refill (TraceIO::refill > 0): instead of tracing a claimed batch of
-// 32 rays to its end, the warp hands new rays to its idle lanes whenever at
-// least `refill` of them are idle (one claim for all of them), keeping the
-// lanes busy while long rays finish.  Pays on incoherent rays, whose walks
-// differ most in length (diffuse secondaries: -11% trace time); costs ~2% on
-// coherent camera rays, so it is a tuning choice.
+// Whether the 32 rays from `base` walk alike: origins within a few cells of the
+// first ray's and directions within a narrow cone of its (camera rays, shadow
+// rays of one surface).  Slots without a shadow ray (tfar < 0) count as alike.
+// One component at a time: the lanes' walks are live around it.
+static __device__ __noinline__ bool chunk_alike(float cx, float cy, float cz, const float4* rays, int32_t n, int32_t base) {
+    const int32_t r = min(base + (int32_t)(threadIdx.x & 31), n - 1);
+    const float* __restrict__ q = reinterpret_cast<const float*>(rays + 2 * (int64_t)r);
+    const float cell[3] = {cx, cy, cz};
+    bool alike = true;
+    float off = 0.0f, len = 0.0f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float o = __ldg(q + a), d = __ldg(q + 4 + a);
+        const float o0 = __shfl_sync(FULL, o, 0), d0 = __shfl_sync(FULL, d, 0);
+        if (!(fabsf(o - o0) <= kChunkCells * cell[a])) alike = false;
+        off += fabsf(d - d0);
+        len += fabsf(d0);
+    }
+    return __all_sync(FULL, (alike && off <= kChunkCone * len) || __ldg(q + 7) < 0.0f);
+}
+__device__ __forceinline__ bool chunk_coherent(const SParams& P, const TraceIO& io, int32_t base) {
+    return chunk_alike(P.cell[0], P.cell[1], P.cell[2], io.rays, (int32_t)io.n, base);
+}
+
+// Lane refill for incoherent rays: instead of tracing a claimed batch of 32 to
+// its end, the warp hands new rays to its idle lanes whenever at least
+// io.refill of them are idle (one claim for all of them), keeping the lanes
+// busy while long rays finish.  Starts on the 32 rays at `chunk` and goes on to
+// the launch's last ray.
 template <int MODE, int ER>
 __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& s, const TraceIO& io, Lane& L,
-                                             uint32_t& cells, uint32_t& tests, uint32_t& started) {
+                                             unsigned long long chunk, uint32_t& cells, uint32_t& tests,
+                                             uint32_t& started) {
     const int lane = threadIdx.x & 31;
-    bool active = false, exhausted = false;
-    int32_t heavy = io.heavy, work_cap = kNoHeavy;
+    bool active = false, exhausted = false, first = true;
     for (;;) {
         const unsigned idle = __ballot_sync(FULL, !active);
         if (!exhausted && ((int)__popc(idle) >= io.refill || idle == FULL)) {
             const unsigned need = (unsigned)__popc(idle);
-            unsigned long long b = 0;
-            if (lane == 0) b = atomicAdd(io.counter, (unsigned long long)need);
-            b = __shfl_sync(FULL, b, 0);
+            unsigned long long b = chunk;
+            if (!first) {
+                if (lane == 0) b = atomicAdd(io.counter, (unsigned long long)need);
+                b = __shfl_sync(FULL, b, 0);
+            }
+            first = false;
             if ((long long)(b + need) >= io.n) exhausted = true;
             if (!active) {
                 const long long ray = (long long)b + __popc(idle & ((1u << lane) - 1u));
                 if (ray < io.n) {
                     L.ray = (int32_t)ray;
-                    heavy = io.heavy;
-                    work_cap = heavy < kNoHeavy / (kHeavyWorkMult + 1) && kHeavyWorkMult > 0 ? heavy * kHeavyWorkMult
-                                                                                             : kNoHeavy;
+                    set_deferral(L, io.heavy);
                     ++started;
                     if (start_ray<MODE>(P, io, L, L.ray)) {
                         active = true;
@@ -750,8 +827,7 @@ __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& 
             if (exhausted) break;
             continue;
         }
-        bool fin = active &&
-                   advance<MODE, ER>(P, L, s.offsets, s.ids, s.tris, s.wald, s.occ, s.crec, heavy, work_cap, cells, tests);
+        bool fin = advance_two<MODE, ER>(P, L, s, active, cells, tests);
         if (io.defer) {
             const bool d = fin && L.id == kDeferred;
             const unsigned m = __ballot_sync(FULL, d);
@@ -767,8 +843,7 @@ __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& 
                                                    L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
                         active = false;
                     } else {
-                        heavy = kNoHeavy;
-                        work_cap = kNoHeavy;
+                        set_deferral(L, kNoHeavy);
                         L.id = -1;
                     }
                     fin = false;
@@ -780,24 +855,28 @@ __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& 
 }
 
 template <int MODE, bool COUNT, int ER, int TPB>
-__global__ void __launch_bounds__(TPB, GRIDRT_TRACE_MIN_BLOCKS * 128 / TPB) trace_kernel(SceneView s, TraceIO io) {
+__global__ void __launch_bounds__(TPB, trace_min_blocks(MODE, TPB)) trace_kernel(SceneView s, TraceIO io) {
     pdl_begin();
     __shared__ SParams P;
     load_sparams(s.params, P);
     const int lane = threadIdx.x & 31;
     Lane L;
     uint32_t cells = 0, tests = 0, started = 0;
-    if (io.refill > 0) {
-        trace_refill<MODE, ER>(P, s, io, L, cells, tests, started);
-    } else {
-        for (;;) {
-            // the warp claims the next 32 consecutive rays and traces them to the end
-            unsigned long long b = 0;
-            if (lane == 0) b = atomicAdd(io.counter, 32ull);
-            b = __shfl_sync(FULL, b, 0);
-            if ((long long)b >= io.n) break;
-            trace_batch32<MODE, ER>(P, s, io, L, (long long)b, cells, tests, started);
+    unsigned long long b = 0;
+    if (lane == 0) b = atomicAdd(io.counter, 32ull);
+    b = __shfl_sync(FULL, b, 0);
+    // the warp traces 32 consecutive rays to the end and claims the next 32;
+    // with lane refill, from the first 32 that are not alike on, it hands out
+    // the launch's rays lane by lane
+    constexpr bool kArrays = MODE == MODE_NEAREST || MODE == MODE_ANY;
+    while ((long long)b < io.n) {
+        if (io.refill > 0 && !(kArrays && chunk_coherent(P, io, (int32_t)b))) {
+            trace_refill<MODE, ER>(P, s, io, L, b, cells, tests, started);
+            break;
         }
+        trace_batch32<MODE, ER>(P, s, io, L, (long long)b, cells, tests, started);
+        if (lane == 0) b = atomicAdd(io.counter, 32ull);
+        b = __shfl_sync(FULL, b, 0);
     }
     if (COUNT) flush_counters(io.ctr, started, cells, tests);
 }
@@ -1060,7 +1139,7 @@ __global__ void __launch_bounds__(128, GRIDRT_GROUP_MIN_BLOCKS) trace_group_kern
             if (exhausted) break;
             continue;
         }
-        const bool any = MODE == MODE_ANY || (MODE == MODE_FRAME && L.tmax > -kFltMax);
+        const bool any = any_hit_phase<MODE>(L);
         GroupOut r = group_batch<G>(P, s, L, sg, busy, any, busy ? todo : 0, thr);
         todo = G;
         const bool hand = busy && r.step == GROUP_LIST;
@@ -1367,7 +1446,7 @@ __global__ void __launch_bounds__(kHugeThreads, GRIDRT_HUGE_MIN_BLOCKS) trace_hu
         // one walk, or for a MODE_FRAME camera ray two: its own, then from
         // its start the shadow ray every thread sets up from the hit
         for (int phase = 0; phase < 2; ++phase) {
-            block_walk(P, s, L, done, MODE == MODE_ANY || (MODE == MODE_FRAME && L.tmax > -kFltMax), cells, tests,
+            block_walk(P, s, L, done, any_hit_phase<MODE>(L), cells, tests,
                        red_t, red_id, &stage, io.counter + 7);
             if (!finish_ray<MODE>(io, P, s, L, threadIdx.x == 0)) break;
             done = false;

@@ -481,11 +481,12 @@ rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, const rtg_req
  *                        Costs 19 MB of device memory per scene (the passes' ray queues).
  *   RTG_TUNE_HEAVY_LANES lanes that trace one deferred ray together: 4, 8, 16, 32 (default)
  *   RTG_TUNE_REFILL      n in 1..32: a warp hands new rays to its idle lanes whenever at least
- *                        n are idle, instead of finishing each batch of 32 rays first (pays on
- *                        incoherent rays: +50 to +65% on random in-box rays at 16; 8 gains a
- *                        little more there and costs ~5% on camera rays); 0 off.  Unset, it is
- *                        16 for rays given as arrays (nearest, any, batches) and off for camera
- *                        and frame traces, whose lanes follow a camera ray with its shadow ray
+ *                        n are idle, instead of finishing each batch of 32 rays first (rays
+ *                        given as arrays: only from the first 32 consecutive rays that are not
+ *                        alike in origin and direction on; 4 M random in-box rays take 3.8 ms
+ *                        without, 2.2 ms at 8); 0 off.  Unset, it is 8 for rays given as arrays
+ *                        (nearest, any, batches) and off for camera and frame traces, whose
+ *                        lanes follow a camera ray with its shadow ray
  *   RTG_TUNE_BLOCK       threads per block of the one-lane trace launch: 64, 128 (default) or 256
  *                        (every block size keeps 64 registers a thread and 32 warps an SM)
  *   RTG_TUNE_LANES       lanes that trace each ray from its start: 1 (one ray a lane, the long
