@@ -325,42 +325,86 @@ __device__ __forceinline__ float3 load_vert(const float* __restrict__ verts, int
     return make_float3(__ldg(q), __ldg(q + 1), __ldg(q + 2));
 }
 
-// Enumerates every (cell, triangle) reference of the warp's 32 triangles, 32
-// references per step, and calls emit(cell, tri, active) on every lane.
-template <class Emit>
-__device__ __forceinline__ void warp_expand(const Lite& L, const float* __restrict__ verts,
-                                            const int32_t* __restrict__ idx, int64_t ntris, int64_t base,
-                                            GridParams* p, BuildWork* w, Emit&& emit) {
-    const int lane = threadIdx.x & 31;
-    const int64_t t = base + lane;
-    int32_t lo[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
-    uint32_t cnt = 0;
-    if (t < ntris) {
-        const int32_t i0 = __ldg(idx + 3 * t), i1 = __ldg(idx + 3 * t + 1), i2 = __ldg(idx + 3 * t + 2);
-        const float3 v0 = load_vert(verts, i0), v1 = load_vert(verts, i1), v2 = load_vert(verts, i2);
-        int32_t hi[3];
-        tri_box_range(L, v0, v1, v2, lo, hi);
-        bool ok = true;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            ok = ok && lo[d] >= 0 && hi[d] < L.res[d] && lo[d] <= hi[d];
-            ext[d] = hi[d] - lo[d] + 1;
-        }
-        if (ok) {
-            cnt = (uint32_t)ext[0] * (uint32_t)ext[1] * (uint32_t)ext[2];
+// A triangle's cells, one after the other (x fastest), for a lane that lists
+// its own triangle.
+struct CellCursor {
+    int32_t c;              // current cell
+    int32_t ex, ey, xi, yi; // extent along x and y, cells left in the row and rows left in the slab
+    int32_t row, slab;      // steps from a row's, and a slab's, last cell to the next one's first
+};
+__device__ __forceinline__ CellCursor cell_cursor(const Lite& L, const int32_t lo[3], const int32_t ext[3]) {
+    CellCursor q;
+    const int32_t nx = L.res[0], nxy = L.res[0] * L.res[1];
+    q.c = lo[0] + lo[1] * nx + lo[2] * nxy;
+    q.ex = q.xi = ext[0];
+    q.ey = q.yi = ext[1];
+    q.row = nx - ext[0] + 1;
+    q.slab = nxy - (ext[1] - 1) * nx - ext[0] + 1;
+    return q;
+}
+__device__ __forceinline__ int32_t next_cell(CellCursor& q) {
+    const int32_t c = q.c;
+    if (--q.xi) {
+        ++q.c;
+    } else {
+        q.xi = q.ex;
+        if (--q.yi) {
+            q.c += q.row;
         } else {
-            raise_status(p, w, ST_BAD_RANGE);
-            ext[0] = ext[1] = ext[2] = 1;
+            q.yi = q.ey;
+            q.c += q.slab;
         }
     }
-    unsigned long long incl = cnt;
+    return c;
+}
+
+// The cells of a warp's triangles are listed either by each lane for itself,
+// ~10 instructions a cell for as long as the longest lane, or 32 references a
+// step over the whole warp, ~130 instructions a step (owner search, division,
+// __match_any_sync) with one atomic for the references that share a cell.  A
+// lane lists its own when the warp's longest triangle has less than a third of
+// its references (the fewer instructions), unless more than 20 triangles have
+// one or two: those of a dense cluster share a few cells, and un-merged
+// atomics on one address queue up (skewed scene, count pass 76 -> 131 us).
+// A million triangles, 25 M references: count pass 171 -> 130 us.
+__device__ __forceinline__ bool lanes_list_own(uint32_t cnt, unsigned long long total) {
+    const uint32_t most = __reduce_max_sync(FULL, cnt);
+    return most >= 4 && 3ull * most < total && __popc(__ballot_sync(FULL, cnt <= 2)) <= 20;
+}
+
+// Range and cell count of triangle t (count 0 past the end or outside the
+// grid, the latter with ok = false).
+__device__ __forceinline__ uint32_t tri_cells(const Lite& L, const float* __restrict__ verts,
+                                              const int32_t* __restrict__ idx, int64_t ntris, int64_t t, int32_t lo[3],
+                                              int32_t ext[3], bool& ok) {
+    ok = true;
+    lo[0] = lo[1] = lo[2] = 0;
+    ext[0] = ext[1] = ext[2] = 1;
+    if (t >= ntris) return 0;
+    const int32_t i0 = __ldg(idx + 3 * t), i1 = __ldg(idx + 3 * t + 1), i2 = __ldg(idx + 3 * t + 2);
+    const float3 v0 = load_vert(verts, i0), v1 = load_vert(verts, i1), v2 = load_vert(verts, i2);
+    int32_t hi[3];
+    tri_box_range(L, v0, v1, v2, lo, hi);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned long long y = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += y;
+    for (int d = 0; d < 3; ++d) {
+        ok = ok && lo[d] >= 0 && hi[d] < L.res[d] && lo[d] <= hi[d];
+        ext[d] = hi[d] - lo[d] + 1;
     }
-    const unsigned long long total = __shfl_sync(FULL, incl, 31);
-    const unsigned long long excl = incl - cnt;
+    if (!ok) {
+        ext[0] = ext[1] = ext[2] = 1;
+        return 0;
+    }
+    return (uint32_t)ext[0] * (uint32_t)ext[1] * (uint32_t)ext[2];
+}
+
+// Enumerates every (cell, triangle) reference of the warp's 32 triangles, 32
+// references per step, and calls emit(cell, lane of the triangle, active) on
+// every lane.
+template <class Emit>
+__device__ __forceinline__ void warp_expand(const Lite& L, const int32_t lo[3], const int32_t ext[3],
+                                            unsigned long long incl, unsigned long long excl,
+                                            unsigned long long total, Emit&& emit) {
+    const int lane = threadIdx.x & 31;
     for (unsigned long long r0 = 0; r0 < total; r0 += 32) {
         const unsigned long long r = r0 + lane;
         const bool active = r < total;
@@ -383,9 +427,17 @@ __device__ __forceinline__ void warp_expand(const Lite& L, const float* __restri
         const int32_t y = ly + (int32_t)(rest % (uint32_t)ey);
         const int32_t z = lz + (int32_t)(rest / (uint32_t)ey);
         const int32_t cell = active ? (x + y * L.res[0] + z * L.res[0] * L.res[1]) : -1;
-        emit(cell, (int32_t)(base + j), active);
+        emit(cell, j, active);
     }
-    if (lane == 0 && total) atomicAdd(reinterpret_cast<unsigned long long*>(&p->nrefs), total);
+}
+
+__device__ __forceinline__ unsigned long long warp_inclusive(unsigned long long v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(FULL, v, o);
+        if ((int)(threadIdx.x & 31) >= o) v += y;
+    }
+    return v;
 }
 
 __device__ __forceinline__ void count_body(const float* __restrict__ verts, const int32_t* __restrict__ idx,
@@ -409,7 +461,18 @@ __device__ __forceinline__ void count_body(const float* __restrict__ verts, cons
     }
     __syncthreads();
     for (int64_t base = warp * 32; base < ntris; base += nwarps * 32) {
-        warp_expand(L, verts, idx, ntris, base, p, w, [&](int32_t cell, int32_t, bool active) {
+        int32_t lo[3], ext[3];
+        bool ok;
+        const uint32_t cnt = tri_cells(L, verts, idx, ntris, base + lane, lo, ext, ok);
+        if (!ok) raise_status(p, w, ST_BAD_RANGE);
+        const unsigned long long incl = warp_inclusive(cnt), total = __shfl_sync(FULL, incl, 31);
+        if (lane == 0 && total) atomicAdd(reinterpret_cast<unsigned long long*>(&p->nrefs), total);
+        if (lanes_list_own(cnt, total)) {
+            CellCursor q = cell_cursor(L, lo, ext);
+            for (uint32_t i = 0; i < cnt; ++i) atomicAdd(&counts[next_cell(q)], 1);
+            continue;
+        }
+        warp_expand(L, lo, ext, incl, incl - cnt, total, [&](int32_t cell, int, bool active) {
             const unsigned peers = __match_any_sync(FULL, cell);
             const int leader = __ffs(peers) - 1;
             if (active && lane == leader) {
@@ -440,62 +503,43 @@ __global__ void __launch_bounds__(256) count_kernel(BuildArgs one, const BuildAr
     }
 }
 
+// Lanes list their own triangles' references while every triangle has a
+// resident thread (`own`): each claim waits for its atomic's return, and the
+// merged claims of the warp-wide listing are the fewer once the passes fill the
+// GPU (500 / 65,536 / 102,400 / 1,000,000 triangles: 17.6 -> 8, 13.3 -> 9.8,
+// 10.3 -> 8.6, but 182 -> 212 us).
 __device__ __forceinline__ void scatter_body(const float* __restrict__ verts, const int32_t* __restrict__ idx,
                                                       int64_t ntris, GridParams* p, int32_t* __restrict__ cursor,
-                                                      int32_t* __restrict__ ids, unsigned vbx, unsigned vgx) {
+                                                      int32_t* __restrict__ ids, int sms, unsigned vbx, unsigned vgx) {
     if (p->status & (ST_CELL_CAP | ST_AMBIGUOUS | ST_TOO_BIG | ST_REF_CAP)) return;
     Lite L;
     load_lite(p, L);
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)vbx * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)vgx * blockDim.x) >> 5;
+    const bool own = ntris <= 2048ll * sms;
     for (int64_t base = warp * 32; base < ntris; base += nwarps * 32) {
-        const int64_t t = base + lane;
-        int32_t lo[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
-        uint32_t cnt = 0;
-        if (t < ntris) {
-            const int32_t i0 = __ldg(idx + 3 * t), i1 = __ldg(idx + 3 * t + 1), i2 = __ldg(idx + 3 * t + 2);
-            const float3 v0 = load_vert(verts, i0), v1 = load_vert(verts, i1), v2 = load_vert(verts, i2);
-            int32_t hi[3];
-            tri_box_range(L, v0, v1, v2, lo, hi);
-            bool ok = true;
+        int32_t lo[3], ext[3];
+        bool ok;
+        const uint32_t cnt = tri_cells(L, verts, idx, ntris, base + lane, lo, ext, ok);
+        const unsigned long long incl = warp_inclusive(cnt), total = __shfl_sync(FULL, incl, 31);
+        if (own && lanes_list_own(cnt, total)) {
+            // four cursors claimed before the first is used: the atomics'
+            // round trips to L2 overlap
+            CellCursor q = cell_cursor(L, lo, ext);
+            const int32_t t = (int32_t)(base + lane);
+            uint32_t i = 0;
+            for (; i + 4 <= cnt; i += 4) {
+                int32_t at[4];
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                ok = ok && lo[d] >= 0 && hi[d] < L.res[d] && lo[d] <= hi[d];
-                ext[d] = hi[d] - lo[d] + 1;
+                for (int u = 0; u < 4; ++u) at[u] = atomicSub(&cursor[next_cell(q)], 1) - 1;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) ids[at[u]] = t;
             }
-            if (ok) cnt = (uint32_t)ext[0] * (uint32_t)ext[1] * (uint32_t)ext[2];
-            else ext[0] = ext[1] = ext[2] = 1;
+            for (; i < cnt; ++i) ids[atomicSub(&cursor[next_cell(q)], 1) - 1] = t;
+            continue;
         }
-        unsigned long long incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned long long y = __shfl_up_sync(FULL, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const unsigned long long total = __shfl_sync(FULL, incl, 31);
-        const unsigned long long excl = incl - cnt;
-        for (unsigned long long r0 = 0; r0 < total; r0 += 32) {
-            const unsigned long long r = r0 + lane;
-            const bool active = r < total;
-            int lo_ = 0, hi_ = 31;
-#pragma unroll
-            for (int s = 0; s < 5; ++s) {
-                const int mid = (lo_ + hi_) >> 1;
-                const unsigned long long im = __shfl_sync(FULL, incl, mid);
-                if (im > r) hi_ = mid; else lo_ = mid + 1;
-            }
-            const int j = lo_;
-            const unsigned long long ex_j = __shfl_sync(FULL, excl, j);
-            const int32_t lx = __shfl_sync(FULL, lo[0], j), ly = __shfl_sync(FULL, lo[1], j),
-                          lz = __shfl_sync(FULL, lo[2], j);
-            const int32_t ex = __shfl_sync(FULL, ext[0], j), ey = __shfl_sync(FULL, ext[1], j);
-            const uint32_t l = (uint32_t)(r - ex_j);
-            const uint32_t rest = l / (uint32_t)ex;
-            const int32_t x = lx + (int32_t)(l - rest * (uint32_t)ex);
-            const int32_t y = ly + (int32_t)(rest % (uint32_t)ey);
-            const int32_t z = lz + (int32_t)(rest / (uint32_t)ey);
-            const int32_t cell = active ? (x + y * L.res[0] + z * L.res[0] * L.res[1]) : -1;
+        warp_expand(L, lo, ext, incl, incl - cnt, total, [&](int32_t cell, int j, bool active) {
             const unsigned peers = __match_any_sync(FULL, cell);
             const int leader = __ffs(peers) - 1;
             const int g = __popc(peers);
@@ -504,7 +548,7 @@ __device__ __forceinline__ void scatter_body(const float* __restrict__ verts, co
             if (active && lane == leader) old = atomicSub(&cursor[cell], g);
             old = __shfl_sync(FULL, old, leader);
             if (active) ids[old - g + rank] = (int32_t)(base + j);
-        }
+        });
     }
 }
 
@@ -515,10 +559,10 @@ __global__ void __launch_bounds__(256) scatter_kernel(BuildArgs one, const Build
     if (MULTI) {
         const int t = block_task(first, ntasks);
         const BuildArgs& a = many[t];
-        scatter_body(a.verts, a.idx, a.ntris, a.params, a.offsets, a.ids, blockIdx.x - (unsigned)first[t], (unsigned)(first[t + 1] - first[t]));
+        scatter_body(a.verts, a.idx, a.ntris, a.params, a.offsets, a.ids, a.num_sms, blockIdx.x - (unsigned)first[t], (unsigned)(first[t + 1] - first[t]));
     } else {
         const BuildArgs& a = one;
-        scatter_body(a.verts, a.idx, a.ntris, a.params, a.offsets, a.ids, blockIdx.x, gridDim.x);
+        scatter_body(a.verts, a.idx, a.ntris, a.params, a.offsets, a.ids, a.num_sms, blockIdx.x, gridDim.x);
     }
 }
 
@@ -547,6 +591,20 @@ __device__ __forceinline__ int64_t block_sum_i64(int64_t v, int64_t* sh) {
     return s;
 }
 
+// A thread's SCAN_ITEMS counts from cell b on (a multiple of SCAN_ITEMS; the
+// offsets are 16-byte aligned), 0 past the grid.
+static_assert(SCAN_ITEMS == 4, "one int4 a thread");
+__device__ __forceinline__ void load_counts(const int32_t* __restrict__ counts, int64_t b, int64_t C,
+                                            int32_t v[SCAN_ITEMS]) {
+    if (b + SCAN_ITEMS <= C) {
+        const int4 q = *reinterpret_cast<const int4*>(counts + b);
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < SCAN_ITEMS; ++i) v[i] = b + i < C ? counts[b + i] : 0;
+    }
+}
+
 __device__ __forceinline__ void scan_reduce_body(const int32_t* __restrict__ counts,
                                                                    const GridParams* __restrict__ p,
                                                                    int64_t* __restrict__ tile_sums, unsigned vbx, unsigned vgx) {
@@ -556,10 +614,11 @@ __device__ __forceinline__ void scan_reduce_body(const int32_t* __restrict__ cou
     __shared__ int64_t sh[33];
     for (int64_t tile = vbx; tile < ntiles; tile += vgx) {
         const int64_t b = tile * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+        int32_t v[SCAN_ITEMS];
+        load_counts(counts, b, C, v);
         int64_t s = 0;
 #pragma unroll
-        for (int i = 0; i < SCAN_ITEMS; ++i)
-            if (b + i < C) s += counts[b + i];
+        for (int i = 0; i < SCAN_ITEMS; ++i) s += v[i];
         s = block_sum_i64(s, sh);
         if (threadIdx.x == 0) tile_sums[tile] = s;
     }
@@ -584,6 +643,8 @@ __device__ __forceinline__ int sort_class(int32_t n) {
     return n <= SORT_TINY_MAX ? 0 : (n <= SORT_SMALL_MAX ? 3 : (n <= SORT_MED_MAX ? 1 : 2));
 }
 
+// Bound by its barriers and atomics, not by the 8 bytes a cell: 6 M cells take
+// 42 us (65 with four scalar loads a thread and an atomicMax a warp).
 // In-place inclusive scan of each tile plus the sum of the tiles before it
 // (each block adds those tile sums itself); queues cells that hold two or
 // more triangles for the segmented sort.  The block of the last tile writes
@@ -615,19 +676,17 @@ __device__ __forceinline__ void scan_down_body(int32_t* __restrict__ counts, Gri
 #pragma unroll 4
     for (int64_t j = threadIdx.x; j < t0; j += blockDim.x) before += tile_sums[j];
     int64_t prefix = block_sum_i64(before, shs);
+    int32_t vmax = 0;
     for (int64_t tile = t0; tile < t1; ++tile) {
         const int64_t b = tile * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
         int32_t v[SCAN_ITEMS];
+        load_counts(counts, b, C, v);
         int64_t s = 0;
-        int32_t vmax = 0;
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; ++i) {
-            v[i] = (b + i < C) ? counts[b + i] : 0;
             s += v[i];
             vmax = max(vmax, v[i]);
         }
-        vmax = (int32_t)__reduce_max_sync(FULL, (unsigned)vmax);
-        if (lane == 0 && vmax > 0) atomicMax(&p->max_list, (unsigned)vmax);
         int64_t x = s;
         for (int o = 1; o < 32; o <<= 1) {
             int64_t y = __shfl_up_sync(FULL, x, o);
@@ -722,11 +781,12 @@ __device__ __forceinline__ void scan_down_body(int32_t* __restrict__ counts, Gri
         uint32_t jm = qbase[1] + wq[wid][1] + ((excl >> 8) & 255u);
         uint32_t jl = qbase[2] + wq[wid][2] + ((excl >> 16) & 255u);
         uint32_t jw = qbase[3] + wq[wid][3] + (excl >> 24);
+        int32_t ends[SCAN_ITEMS];
 #pragma unroll
         for (int i = 0; i < SCAN_ITEMS; ++i) {
             if (b + i < C) {
                 run += v[i];
-                counts[b + i] = (int32_t)run;
+                ends[i] = (int32_t)run;
                 const int32_t n = v[i];
                 if (n >= 2) {
                     if (n <= SORT_TINY_MAX) {
@@ -749,6 +809,22 @@ __device__ __forceinline__ void scan_down_body(int32_t* __restrict__ counts, Gri
                 }
             }
         }
+        if (b + SCAN_ITEMS <= C) {
+            *reinterpret_cast<int4*>(counts + b) = make_int4(ends[0], ends[1], ends[2], ends[3]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < SCAN_ITEMS; ++i)
+                if (b + i < C) counts[b + i] = ends[i];
+        }
+    }
+    // the longest list, one atomic a block (one a warp and tile were 47,000
+    // to one address at 6 M cells)
+    vmax = (int32_t)__reduce_max_sync(FULL, (unsigned)vmax);
+    if (lane == 0) wq[wid][0] = (uint32_t)vmax;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < SCAN_THREADS / 32; ++i) vmax = max(vmax, (int32_t)wq[i][0]);
+        if (vmax > 0) atomicMax(&p->max_list, (unsigned)vmax);
     }
 }
 
