@@ -124,6 +124,7 @@ BuildArgs make_args(rtg_scene s, int32_t k, bool skip_bbox) {
     a.crec = s->tune.cell_records ? s->d_crec : nullptr;
     a.scratch = s->d_scratch;
     a.ref_cap = ref_capacity(s);
+    a.csph = s->csph_cap >= a.ref_cap ? s->d_csph : nullptr;
     a.tile_sums = s->d_tiles;
     a.q_small = s->d_qs;
     a.q_med = s->d_qm;
@@ -201,7 +202,7 @@ rtg_status enqueue_build(rtg_scene s, int32_t k, bool skip_bbox, cudaStream_t st
     if (skip_bbox)
         CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(s->d_work) + offsetof(BuildWork, nsort), 0,
                                  sizeof(BuildWork::nsort), st));
-    launch_build(make_args(s, k, skip_bbox), st, s->have_fork ? &s->fork : nullptr);
+    s->csph_built = launch_build(make_args(s, k, skip_bbox), st, s->have_fork ? &s->fork : nullptr);
     CUDA_TRY(cudaGetLastError());
     return RTG_OK;
 }
@@ -252,6 +253,7 @@ SceneView scene_view(rtg_scene s) {
     v.ids = s->d_ids;
     v.occ = s->d_occ;
     v.crec = (s->tune.cell_records && s->crec_built) ? s->d_crec : nullptr;
+    v.csph = s->csph_built ? s->d_csph : nullptr;
     v.tris = s->d_tris;
     v.wald = s->d_wald;
     return v;
@@ -361,6 +363,7 @@ rtg_status rtg_scene_destroy(rtg_scene s) {
     cudaFree(s->d_ids);
     cudaFree(s->d_scratch);
     cudaFree(s->d_crec);
+    cudaFree(s->d_csph);
     cudaFree(s->d_tiles);
     cudaFree(s->d_qs);
     cudaFree(s->d_qm);
@@ -599,6 +602,12 @@ rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) {
         }
         if (p.status & ST_BAD_RANGE)
             return fail(RTG_INVALID_GEOMETRY, "non-finite vertex or triangle outside the grid");
+        // a scene with crowded lists keeps their triangles' bounding spheres:
+        // make room the first time, and build once more with them
+        if (p.max_list > (uint32_t)kSplitRefs && s->csph_cap < ref_capacity(s) && attempt < 4) {
+            if (grow(s->d_csph, s->csph_cap, ref_capacity(s)) == cudaSuccess) continue;
+            cudaGetLastError();   // without them the block-per-ray pass reads the records
+        }
         s->hp = p;
         s->built = true;
         s->crec_built = s->tune.cell_records != 0;
@@ -1083,6 +1092,7 @@ rtg_status rtg_batch_build_async(rtg_batch b, void* stream) {
         if (rc == RTG_OK) rc = apply_staged(sc, st);
         if (rc) return rc;
         sc->crec_built = sc->tune.cell_records != 0;   // this build writes them
+        sc->csph_built = false;                        // and no spheres (batch traces have no block-per-ray pass)
     }
     rtg_status rc = batch_upload_build(b, st, false);
     if (rc == RTG_OK) rc = batch_upload_views(b, st, false);

@@ -30,6 +30,7 @@
 
 #include <climits>
 #include <cooperative_groups.h>
+#include <cuda_fp16.h>
 
 namespace gridrt {
 
@@ -992,9 +993,6 @@ __global__ void __launch_bounds__(512) sort_medium_kernel(BuildArgs one, const B
 // one shared-memory bit per id (per id chunk, from a scratch copy, when the
 // scene has more triangles than the bitmap has bits), then the set bits
 // written back in order.
-// Lists above kSplitRefs entries of a single-scene build whose ids fit one
-// bitmap span are sorted by sort_split_kernel, the rest by sort_large.
-static constexpr int32_t kSplitRefs = SORT_BLOCK_MAX;
 static constexpr int kSplitBlocks = 8;   // blocks of a list's cluster (the portable maximum)
 
 __device__ __forceinline__ void sort_large_body(const int32_t* __restrict__ offsets,
@@ -1149,6 +1147,36 @@ __global__ void __launch_bounds__(1024) sort_large_kernel(BuildArgs one, const B
     }
 }
 
+// Bounding sphere of what RayTriIntersection::hitWald can accept of a triangle:
+// {centre, two halves}, radius r0 + w x 256u (|origin|_1 + 2 |x|_1) for a ray
+// whose accepted points x lie about a cell the triangle overlaps, u = 2^-24.
+// The barycentrics of hitWald are off by at most 16u |b|_1 H, H = |origin|_1 +
+// 2 |vertex|_1, |b|_1 the sum of a row's |coefficients| (and their scale by 4u
+// |b|_1 ext), so an accepted point lies within 64u (q + 1) H of the triangle on
+// each axis, q = (|b|_1 + |c|_1) ext, ext the triangle's extent; twice that for
+// the Euclidean distance, and once more for the sphere test's own rounding.
+// w = q + 1; vertices lie within 6 r0 of the cell, which r0 takes in.  Both
+// halves are rounded up; what overflows or is not a number is always met.
+__device__ __forceinline__ float4 hit_sphere(const float4& A, const float4& B, const float4& C) {
+    const float bx = C.x, by = C.y, bz = C.z, cx = B.x, cy = B.y, cz = B.z;   // v2 - v0, v1 - v0
+    const float mx = (bx + cx) * (1.0f / 3.0f), my = (by + cy) * (1.0f / 3.0f), mz = (bz + cz) * (1.0f / 3.0f);
+    auto d2 = [&](float x, float y, float z) {
+        x -= mx;
+        y -= my;
+        z -= mz;
+        return x * x + y * y + z * z;
+    };
+    // the rows' denominator is the normal's largest component; the edges'
+    // components sum to at least the rows' times it
+    const float nx = cy * bz - cz * by, ny = cz * bx - cx * bz, nz = cx * by - cy * bx;
+    const float den = fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz));
+    const float edges = fabsf(bx) + fabsf(by) + fabsf(bz) + fabsf(cx) + fabsf(cy) + fabsf(cz);
+    const float r0 = 1.001f * sqrtf(fmaxf(fmaxf(d2(0.f, 0.f, 0.f), d2(bx, by, bz)), d2(cx, cy, cz)));
+    const float w = 1.0f + edges * (2.0f * r0) / den;          // the extent is at most the diameter
+    const __half2 h = __halves2half2(__float2half_ru(r0 * (1.0f + 256.0f * 12.0f * kRound * w)), __float2half_ru(w));
+    return make_float4(A.x + mx, A.y + my, A.z + mz, __uint_as_float(*reinterpret_cast<const uint32_t*>(&h)));
+}
+
 // A list above kSplitRefs entries, split by triangle id over the
 // kSplitBlocks blocks of a thread-block cluster: block r owns the ids of
 // slice r of [0, ntris) and a shared-memory bitmap of that slice.  Each
@@ -1240,8 +1268,29 @@ __global__ void __launch_bounds__(1024) sort_split_kernel(BuildArgs a) {
             }
         }
         // no block clears its bitmap or republishes its count for the next
-        // list while another may still read them
+        // list while another may still read them; the whole list is written
         cl.sync();
+        if (a.csph) {
+            // the bounding spheres of this block's eighth of the list, four
+            // records' loads in flight a thread
+            for (int32_t i0 = p0 + (int32_t)threadIdx.x; i0 < p1; i0 += kSortLoads * (int32_t)blockDim.x) {
+                float4 A[kSortLoads], B[kSortLoads], C[kSortLoads];
+                int32_t t[kSortLoads];
+#pragma unroll
+                for (int u = 0; u < kSortLoads; ++u) t[u] = a.ids[s + min(i0 + u * (int32_t)blockDim.x, p1 - 1)];
+#pragma unroll
+                for (int u = 0; u < kSortLoads; ++u) {
+                    A[u] = __ldg(a.tris + 3 * (int64_t)t[u]);
+                    B[u] = __ldg(a.tris + 3 * (int64_t)t[u] + 1);
+                    C[u] = __ldg(a.tris + 3 * (int64_t)t[u] + 2);
+                }
+#pragma unroll
+                for (int u = 0; u < kSortLoads; ++u) {
+                    const int32_t i = i0 + u * (int32_t)blockDim.x;
+                    if (i < p1) a.csph[s + i] = hit_sphere(A[u], B[u], C[u]);
+                }
+            }
+        }
     }
 }
 
@@ -1355,7 +1404,7 @@ static cudaError_t launch_cluster_k(void (*kernel)(KArgs...), unsigned grid, uns
 }
 
 template <bool MULTI>
-static void launch_build_impl(const BuildArgs& one, const BuildArgs* many, int ntasks, const BatchGrid& g,
+static bool launch_build_impl(const BuildArgs& one, const BuildArgs* many, int ntasks, const BatchGrid& g,
                               bool skip_bbox, int bitmap_words, cudaStream_t st, const BuildFork* fork = nullptr) {
     count_launches(9);
     const int* f[kBuildKinds];
@@ -1412,6 +1461,7 @@ static void launch_build_impl(const BuildArgs& one, const BuildArgs* many, int n
     if (split) {
         const int clusters = one.num_sms / kSplitBlocks > 0 ? one.num_sms / kSplitBlocks : 1;
         const int64_t words = ((one.ntris + kSplitBlocks - 1) / kSplitBlocks + 31) / 32 + 1;
+        if (rec_side && one.csph) cudaStreamWaitEvent(sl, fork->rec_join, 0);   // the spheres are made from the records
         if (launch_cluster_k(sort_split_kernel, (unsigned)(clusters * kSplitBlocks), 1024u, (size_t)words * 4, sl,
                              (unsigned)kSplitBlocks, one) == cudaSuccess) {
             count_launches(1);
@@ -1434,12 +1484,13 @@ static void launch_build_impl(const BuildArgs& one, const BuildArgs* many, int n
         count_launches(1);
         launch_k(cell_records_kernel<MULTI>, g.total[BK_REFS], 256, 0, st, one, many, f[BK_REFS], ntasks);
     }
+    return split && one.csph;
 }
 
-void launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork) {
+bool launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork) {
     BatchGrid g{};
     build_blocks(a, a.num_sms, g.total);
-    launch_build_impl<false>(a, nullptr, 1, g, a.skip_bbox, a.bitmap_words, st, fork);
+    return launch_build_impl<false>(a, nullptr, 1, g, a.skip_bbox, a.bitmap_words, st, fork);
 }
 
 void launch_build_batch(const BuildArgs* d_tasks, int ntasks, const BatchGrid& g, int bitmap_words,

@@ -79,6 +79,7 @@ struct BuildWork {
 static constexpr float kHitEpsilon = 1e-4f;   // src/rtcore/RayTriIntersection.cpp:6
 static constexpr float kRayEpsilon = 2e-4f;   // src/rtcore/Context.cpp:505
 static constexpr float kFltMax = 3.402823466e+38f;
+static constexpr float kRound = 5.9604645e-8f;   // 2^-24: the largest relative error of one float operation
 
 // Sets status bits on the current build and on the sticky word.
 __device__ __forceinline__ void raise_status(GridParams* p, BuildWork* w, uint32_t bits) {

@@ -25,6 +25,7 @@ struct BuildArgs {
     int64_t cell_cap;
     int32_t* ids;          // ref_cap entries
     float4* crec;          // optional: 3 x ref_cap float4, triangle records in cell-list order
+    float4* csph;          // optional: ref_cap float4, bounding spheres of the lists above kSplitRefs, in list order
     int32_t* scratch;      // ref_cap entries
     int64_t ref_cap;
     int64_t* tile_sums;
@@ -35,6 +36,11 @@ struct BuildArgs {
     int32_t bitmap_words;
     int num_sms;
 };
+
+// Lists above kSplitRefs entries of a single-scene build whose ids fit one
+// bitmap span are sorted by sort_split_kernel, which also writes their
+// triangles' bounding spheres; the rest by sort_large.
+static constexpr int32_t kSplitRefs = SORT_BLOCK_MAX;
 
 // Cells per tile of the count scan (tile sums: cell capacity / kScanTile + 2).
 static constexpr int kScanTile = 1024;
@@ -56,7 +62,8 @@ struct BuildFork {
     cudaEvent_t rec_clear;   // the offsets and bitmap cleared (the count pass waits for it)
     cudaEvent_t rec_join;
 };
-void launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork = nullptr);
+// True when the lists above kSplitRefs got their bounding spheres (a.csph).
+bool launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork = nullptr);
 
 // Build kernels by work shape (grid sizing per task).
 enum BuildKind { BK_BBOX = 0, BK_ZERO, BK_TRI, BK_TILE, BK_SSMALL, BK_SMED, BK_SLARGE, BK_REFS, BK_RECS, kBuildKinds };
@@ -84,6 +91,7 @@ struct SceneView {
     const int32_t* ids;
     const uint32_t* occ;
     const float4* crec;    // records in cell-list order, or nullptr (then ids -> tris)
+    const float4* csph;    // bounding spheres of the lists above kSplitRefs in list order, or nullptr
     const float4* tris;
     const float4* wald;    // TriAccel records: the reported t / u / v of a hit (nullptr: from tris)
 };

@@ -183,7 +183,7 @@ extern "C" rtg_status rtg_grid_build_noalloc(const float* d_verts, int64_t nvert
     a.wald = nullptr;  // hit-value records serve only the scene's trace kernels
     a.offsets = d_offsets;
     a.occ = nullptr;   // the occupancy bitmap only serves the scene's trace kernels
-    a.crec = nullptr;
+    a.crec = a.csph = nullptr;
     a.cell_cap = offsets_cap < kMaxCells + 1 ? offsets_cap : kMaxCells + 1;
     a.ids = d_ids;
     a.scratch = reinterpret_cast<int32_t*>(d->arena + kOffScratch);

@@ -43,6 +43,8 @@ struct rtg_scene_s {
     int64_t ids_cap = 0;
     float4* d_crec = nullptr;            // cell-ordered triangle records (tune.cell_records)
     int64_t crec_cap = 0;                // in float4
+    float4* d_csph = nullptr;            // bounding spheres of crowded lists, list order (once a build had such lists)
+    int64_t csph_cap = 0;
     int32_t* d_scratch = nullptr;
     int64_t scratch_cap = 0;
     int64_t* d_tiles = nullptr;
@@ -57,6 +59,7 @@ struct rtg_scene_s {
 
     bool built = false;
     bool crec_built = false;             // the last build wrote cell-ordered records
+    bool csph_built = false;             // the last build wrote the crowded lists' spheres
     int32_t k = 0;
     gridrt::GridParams hp{};   // host copy of the last successful build
 

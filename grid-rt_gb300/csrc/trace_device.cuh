@@ -31,6 +31,8 @@
 #include "common.cuh"
 #include "kernels.h"
 
+#include <cuda_fp16.h>
+
 namespace gridrt {
 
 static constexpr float kChunkCells = 4.0f;   // chunk_coherent: origins, in cells
@@ -924,7 +926,7 @@ __device__ __forceinline__ void resume_at(const SParams& P, Lane& L, int32_t cel
 enum GroupStep : int { GROUP_ON = 0, GROUP_DONE = 1, GROUP_LIST = 2 };
 struct GroupOut {
     int step;
-    int32_t cell, len;        // GROUP_LIST
+    int32_t cell, len, lane;  // GROUP_LIST: the cell, its list's length, the lane that stands on it
     int32_t cells, tests;     // visited and tested by the one-lane walk's count
 };
 
@@ -936,10 +938,11 @@ __device__ __forceinline__ int3 step_signs(const Lane& L) {
 
 // Moves every lane `todo` cells on (its place in the group for a new ray, G
 // after that, 0 to visit the same cells again) and tests the lists of the
-// group's cells.  Called by the whole warp; `busy` is the same for a group.
+// group's cells, but for those of its first `skip` + 1 lanes.  Called by the
+// whole warp; `busy` is the same for a group.
 template <int G>
 __device__ __forceinline__ GroupOut group_batch(const SParams& P, const SceneView& s, Lane& L, const int3& sg,
-                                                bool busy, bool any, int todo, int32_t thr) {
+                                                bool busy, bool any, int todo, int32_t thr, int skip = -1) {
     const int lane = threadIdx.x & 31, gl = lane & (G - 1), g0 = lane & ~(G - 1);
     constexpr unsigned gm = G == 32 ? FULL : ((1u << G) - 1u);
     // dda_step without its exit test: a coordinate that has left the grid
@@ -957,7 +960,7 @@ __device__ __forceinline__ GroupOut group_batch(const SParams& P, const SceneVie
     const bool out = (unsigned)L.x >= (unsigned)P.res[0] || (unsigned)L.y >= (unsigned)P.res[1] ||
                      (unsigned)L.z >= (unsigned)P.res[2] || L.budget <= 0;
     int32_t b = 0, n = 0, c = 0;
-    if (busy && !out) {
+    if (busy && !out && gl > skip) {
         const int32_t w = (L.x >> 2) + (L.y >> 2) * P.bx + (L.z >> 1) * P.bxby;
         if (__ldg(s.occ + w) & occ_bit(L.x, L.y, L.z)) {
             c = L.x + P.res[0] * (L.y + L.z * P.res[1]);
@@ -1033,6 +1036,7 @@ __device__ __forceinline__ GroupOut group_batch(const SParams& P, const SceneVie
     GroupOut r;
     r.cell = __shfl_sync(FULL, c, fh & (G - 1), G);
     r.len = __shfl_sync(FULL, n, fh & (G - 1), G);
+    r.lane = fh;
     r.tests = limit;
     if (hj < G) {
         r.step = GROUP_DONE;
@@ -1050,6 +1054,7 @@ __device__ __forceinline__ GroupOut group_batch(const SParams& P, const SceneVie
         r.step = GROUP_ON;
         r.cells = G;
     }
+    r.cells -= skip + 1;
     return r;
 }
 
@@ -1184,13 +1189,16 @@ __global__ void __launch_bounds__(128, GRIDRT_GROUP_MIN_BLOCKS) trace_group_kern
 }
 
 // Block-per-ray pass over the rays the group pass met at a list above
-// kHugeList (a dense cluster: tens of thousands of triangles in one cell):
-// all threads of the block hold the ray and step the same DDA; each list is
+// kHugeList (a dense cluster: tens of thousands of triangles in one cell).  The
+// block's first warp walks the ray as the group pass does; each long list is
 // split over the block (thread j tests entries j, j + blockDim, ...), each
 // thread keeping the first minimum of its share, and a block reduction takes
 // the minimum t, ties to the earlier entry -- the one-lane walk's result, as
-// in the group pass.  A ray's walk then takes a block's time per list, not a
-// lane's or a group's.
+// in the group pass.  Bound by the longest rays, one block each (several
+// hundred thousand entries), and by their walks between crowded cells.  Lists
+// above kSplitRefs are read as 16-byte bounding spheres: 1,048,576 triangles of
+// skewed density, the passes behind 1024^2 camera rays and their secondaries
+// 420 and 489 -> 240..290 and 270 us, the spheres 25 us of the build's sort.
 #ifndef GRIDRT_HUGE_THREADS
 #define GRIDRT_HUGE_THREADS 256
 #endif
@@ -1229,10 +1237,13 @@ static constexpr int32_t kStageMin = 2 * kHugeThreads;
 static constexpr uint32_t kStageWaitLimit = 1u << 24;
 static_assert(kStageEntries % kHugeThreads == 0 || kHugeThreads % kStageEntries == 0, "stage chunk");
 
+static constexpr int kCand = 512;
 struct Stage {
     float4* buf;          // shared: kStageDepth x kStageEntries x 3 float4
     uint64_t* bar;        // shared: one mbarrier per buffer
     int* off;             // shared: 1 once a wait has run out
+    int32_t* cand;        // shared: candidates of a list's spheres, kCand at most
+    int* cand_n;          // shared: how many there were
     uint32_t phase;       // bit q: the parity of buffer q's next completion
 };
 
@@ -1263,46 +1274,155 @@ __device__ __forceinline__ bool stage_wait(uint64_t* bar, uint32_t parity) {
     return false;
 }
 
-// The block's ray (identical state on every thread) walked to its end:
-// each list split over the block, a block reduction per list.
+// Whether the ray's line meets a list entry's bounding sphere (build.cu
+// hit_sphere; `grow`: 256u (|origin|_1 + 2 |x|_1) of the ray and the cell, dd:
+// |d|^2 and a margin).  19 instructions on 16 bytes: nearly all of a dense
+// cluster's triangles end here.
+__device__ __forceinline__ bool near_sphere(const Lane& L, const float4& q, float grow, float dd) {
+    const float2 rw = __half22float2(*reinterpret_cast<const __half2*>(&q.w));
+    const float r = rw.x + rw.y * grow;
+    const float x = q.x - L.ox, y = q.y - L.oy, z = q.z - L.oz;
+    const float cx = y * L.dz - z * L.dy, cy = z * L.dx - x * L.dz, cz = x * L.dy - y * L.dx;
+    return !(cx * cx + cy * cy + cz * cz > r * r * dd);
+}
+
+// The largest |x|_1 in a cell (and a margin).
+__device__ __forceinline__ float cell_l1(const SParams& P, int32_t cell) {
+    float m = 0.0f;
+    const int32_t nxy = P.res[0] * P.res[1], z = cell / nxy, y = (cell - z * nxy) / P.res[0];
+    const int32_t c[3] = {cell - z * nxy - y * P.res[0], y, z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float lo = P.bmin[a] + P.cell[a] * (float)(c[a] - 1), hi = P.bmin[a] + P.cell[a] * (float)(c[a] + 2);
+        m += fmaxf(fabsf(lo), fabsf(hi));
+    }
+    return m;
+}
+
+// The next larger float (of a finite distance).
+__device__ __forceinline__ float float_above(float x) {
+    const int32_t i = __float_as_int(x);
+    return x == 0.0f ? __int_as_float(1) : __int_as_float(x > 0.0f ? i + 1 : i - 1);
+}
+
+// List entry i from global memory, in any order within the thread's share: of
+// two equal distances the smaller id stays.
+__device__ __forceinline__ void test_listed(Lane& T, const SceneView& s, int32_t i, float hi) {
+    const int32_t t = __ldg(s.ids + i);
+    const float4* __restrict__ r = s.crec ? s.crec + 3 * (int64_t)i : s.tris + 3 * (int64_t)t;
+    const float best = T.best;
+    const int32_t id = T.id;
+    if (id >= 0) T.best = float_above(best);
+    test_tri<MODE_NEAREST>(T, t, __ldg(r), __ldg(r + 1), __ldg(r + 2), hi, s.wald);
+    if (id >= 0 && (T.id == id || (T.best == best && t > id))) {
+        T.best = best;
+        T.id = id;
+    }
+}
+
+// What the block's first warp found next along the ray, for its other threads.
+struct BlockStep {
+    int32_t step, cell, id;
+    float best, hi;
+};
+// Lists longer than this are tested by the whole block.
+static constexpr int32_t kBlockList = kHugeThreads;
+
+// The block's ray walked to its end (the same ray on every thread).  The first
+// warp walks it 32 cells at a time (group_batch) up to the next list above
+// kBlockList; that list is split over the block.  Block-wide steps cell by cell
+// made the rays' walks between crowded cells, each with its own barriers and
+// chain of loads, the pass's time.
 __device__ __forceinline__ void block_walk(const SParams& P, const SceneView& s, Lane& L, bool done, bool any,
                                            uint32_t& cells, uint32_t& tests, float* red_t, int32_t* red_id,
-                                           Stage* st = nullptr, unsigned long long* err = nullptr) {
+                                           BlockStep* bs, Stage* st = nullptr, unsigned long long* err = nullptr) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int32_t nx = P.res[0], nxy = P.res[0] * P.res[1];
-    while (!done) {
-        if (threadIdx.x == 0) ++cells;
-        const int32_t w = (L.x >> 2) + (L.y >> 2) * P.bx + (L.z >> 1) * P.bxby;
-        if (__ldg(s.occ + w) & occ_bit(L.x, L.y, L.z)) {
-            const int32_t c = L.x + L.y * nx + L.z * nxy;
+    if (done) return;
+    const float o1 = fabsf(L.ox) + fabsf(L.oy) + fabsf(L.oz);
+    const float dd = 1.0001f * (L.dx * L.dx + L.dy * L.dy + L.dz * L.dz);
+    const int3 sg = step_signs(L);
+    int todo = lane, skip = -1;
+    for (;;) {
+        if (wid == 0) {
+            GroupOut r;
+            for (;;) {
+                r = group_batch<32>(P, s, L, sg, true, any, todo, kBlockList, skip);
+                if (lane == 0) {
+                    cells += (uint32_t)r.cells;
+                    tests += (uint32_t)r.tests;
+                }
+                if (r.step != GROUP_ON) break;
+                todo = 32;
+                skip = -1;
+            }
+            const float hi = __shfl_sync(FULL, fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon), r.lane & 31);
+            if (lane == 0) *bs = BlockStep{r.step, r.cell, L.id, L.best, hi};
+            todo = 0;         // go on from the cells the lanes stand on, behind this list's
+            skip = r.lane;
+        }
+        __syncthreads();
+        if (bs->step == GROUP_DONE) {
+            L.id = bs->id;
+            L.best = bs->best;
+            __syncthreads();
+            return;
+        }
+        {
+            const int32_t c = bs->cell;
             const int32_t b = __ldg(s.offsets + c), e = __ldg(s.offsets + c + 1);
-            const float hi = fadd(vmin(vmin(L.tMx, L.tMy), L.tMz), kHitEpsilon);
-            if (threadIdx.x == 0) tests += (uint32_t)(e - b);
+            const float hi = bs->hi;
+            if (threadIdx.x == 0) {
+                ++cells;
+                tests += (uint32_t)(e - b);
+            }
             Lane T = L;
             T.id = -1;
-            if (GRIDRT_STAGE && st && s.crec && e - b >= kStageMin && !*st->off) {
+            // a crowded list's entries by their bounding spheres first, when
+            // the scene has them: the candidates (one in 3,000 in a dense
+            // cluster) are queued in shared memory and tested together behind
+            // the list's last chunk -- a warp that tested its own at once
+            // waited for their loads at every step
+            const bool sph = s.csph && e - b > kSplitRefs;
+            const float grow = sph ? 256.0f * kRound * (o1 + 2.0f * cell_l1(P, c)) : 0.0f;
+            if (GRIDRT_STAGE && st && (sph || (s.crec && e - b >= kStageMin)) && !*st->off) {
                 // staged: chunk ch in buffer ch % kStageDepth, the next
                 // kStageDepth - 1 chunks in flight
-                const int32_t nch = (e - b + kStageEntries - 1) / kStageEntries;
+                const float4* __restrict__ src = sph ? s.csph : s.crec;
+                const int32_t quads = sph ? 1 : 3, per = sph ? 3 * kStageEntries : kStageEntries;
+                const int32_t nch = (e - b + per - 1) / per;
+                if (sph) {
+                    if (threadIdx.x == 0) *st->cand_n = 0;
+                    __syncthreads();
+                }
                 if (threadIdx.x == 0) {
                     for (int32_t ch = 0; ch < nch && ch < kStageDepth; ++ch) {
-                        const int32_t cb = b + ch * kStageEntries;
-                        const int32_t cn = e - cb < kStageEntries ? e - cb : kStageEntries;
-                        stage_copy(st->buf + ch * 3 * kStageEntries, s.crec + 3 * (int64_t)cb, (uint32_t)cn * 48u,
-                                   st->bar + ch);
+                        const int32_t cb = b + ch * per;
+                        const int32_t cn = e - cb < per ? e - cb : per;
+                        stage_copy(st->buf + ch * 3 * kStageEntries, src + quads * (int64_t)cb,
+                                   (uint32_t)(cn * quads) * 16u, st->bar + ch);
                     }
                 }
                 for (int32_t ch = 0; ch < nch; ++ch) {
                     const int q = ch % kStageDepth;
-                    const int32_t cb = b + ch * kStageEntries;
-                    const int32_t cn = e - cb < kStageEntries ? e - cb : kStageEntries;
+                    const int32_t cb = b + ch * per;
+                    const int32_t cn = e - cb < per ? e - cb : per;
                     const bool ok = stage_wait(st->bar + q, (st->phase >> q) & 1u);
                     st->phase ^= 1u << q;
                     if (ok) {
                         const float4* sb = st->buf + q * 3 * kStageEntries;
-                        for (int32_t j = (int32_t)threadIdx.x; j < cn; j += kHugeThreads) {
-                            const float4 A = sb[3 * j], B = sb[3 * j + 1], C = sb[3 * j + 2];
-                            test_tri<MODE_NEAREST>(T, __float_as_int(A.w), A, B, C, hi, s.wald);
+                        if (sph) {
+#pragma unroll 3
+                            for (int32_t j = (int32_t)threadIdx.x; j < cn; j += kHugeThreads)
+                                if (near_sphere(L, sb[j], grow, dd)) {
+                                    const int at = atomicAdd(st->cand_n, 1);
+                                    if (at < kCand) st->cand[at] = cb + j;
+                                    else test_listed(T, s, cb + j, hi);
+                                }
+                        } else {
+                            for (int32_t j = (int32_t)threadIdx.x; j < cn; j += kHugeThreads) {
+                                const float4 A = sb[3 * j], B = sb[3 * j + 1], C = sb[3 * j + 2];
+                                test_tri<MODE_NEAREST>(T, __float_as_int(A.w), A, B, C, hi, s.wald);
+                            }
                         }
                     }
                     // every thread is done with buffer q before chunk
@@ -1320,20 +1440,22 @@ __device__ __forceinline__ void block_walk(const SParams& P, const SceneView& s,
                             *st->off = 1;
                             if (err) atomicOr(err, 1ull);
                         }
-                        for (int32_t i = (ok ? cb + cn : cb) + (int32_t)threadIdx.x; i < e; i += kHugeThreads) {
-                            const float4 A = __ldg(s.crec + 3 * (int64_t)i), B = __ldg(s.crec + 3 * (int64_t)i + 1),
-                                         C = __ldg(s.crec + 3 * (int64_t)i + 2);
-                            test_tri<MODE_NEAREST>(T, __float_as_int(A.w), A, B, C, hi, s.wald);
-                        }
+                        for (int32_t i = (ok ? cb + cn : cb) + (int32_t)threadIdx.x; i < e; i += kHugeThreads)
+                            test_listed(T, s, i, hi);
                         __syncthreads();
                         break;
                     }
                     if (threadIdx.x == 0 && ch + kStageDepth < nch) {
-                        const int32_t nb = cb + kStageDepth * kStageEntries;
-                        const int32_t nn = e - nb < kStageEntries ? e - nb : kStageEntries;
-                        stage_copy(st->buf + q * 3 * kStageEntries, s.crec + 3 * (int64_t)nb, (uint32_t)nn * 48u,
-                                   st->bar + q);
+                        const int32_t nb = cb + kStageDepth * per;
+                        const int32_t nn = e - nb < per ? e - nb : per;
+                        stage_copy(st->buf + q * 3 * kStageEntries, src + quads * (int64_t)nb,
+                                   (uint32_t)(nn * quads) * 16u, st->bar + q);
                     }
+                }
+                if (sph) {
+                    // (every chunk ended with a barrier)
+                    const int nc = min(*st->cand_n, kCand);
+                    for (int k = (int)threadIdx.x; k < nc; k += kHugeThreads) test_listed(T, s, st->cand[k], hi);
                 }
             } else if (s.crec) {
                 // two entries a thread per step, both loaded before either is
@@ -1391,13 +1513,8 @@ __device__ __forceinline__ void block_walk(const SParams& P, const SceneView& s,
                 // occluded only below tmax
                 L.best = bt;
                 L.id = (any && !(bt < L.tmax)) ? -1 : bid;
-                done = true;
-                continue;
+                return;
             }
-        }
-        if (dda_step(P, L)) {
-            L.id = -1;
-            done = true;
         }
     }
 }
@@ -1412,13 +1529,16 @@ __global__ void __launch_bounds__(kHugeThreads, GRIDRT_HUGE_MIN_BLOCKS) trace_hu
     extern __shared__ __align__(128) float4 stage_buf[];   // kStageBytes (dynamic)
     __shared__ __align__(8) uint64_t stage_bar[kStageDepth];
     __shared__ int stage_off;
+    __shared__ int32_t cand[kCand];
+    __shared__ int cand_n;
+    __shared__ BlockStep step;
     if (threadIdx.x == 0) {
         for (int q = 0; q < kStageDepth; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(stage_bar + q)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         stage_off = 0;
     }
-    Stage stage{stage_buf, stage_bar, &stage_off, 0u};
+    Stage stage{stage_buf, stage_bar, &stage_off, cand, &cand_n, 0u};
     load_sparams(s.params, P);
     unsigned long long nh = io.counter[3];
     if (nh > (unsigned long long)io.huge_cap) nh = (unsigned long long)io.huge_cap;
@@ -1447,7 +1567,7 @@ __global__ void __launch_bounds__(kHugeThreads, GRIDRT_HUGE_MIN_BLOCKS) trace_hu
         // its start the shadow ray every thread sets up from the hit
         for (int phase = 0; phase < 2; ++phase) {
             block_walk(P, s, L, done, any_hit_phase<MODE>(L), cells, tests,
-                       red_t, red_id, &stage, io.counter + 7);
+                       red_t, red_id, &step, &stage, io.counter + 7);
             if (!finish_ray<MODE>(io, P, s, L, threadIdx.x == 0)) break;
             done = false;
         }
