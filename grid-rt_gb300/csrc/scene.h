@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "../../include/gridrt.h"
 #include "common.cuh"
 #include "kernels.h"
@@ -29,7 +31,7 @@ struct rtg_scene_s {
     int64_t wald_cap = 0;
 
     gridrt::GridParams* d_params = nullptr;
-    gridrt::GridParams* h_params = nullptr;      // pinned mirror
+    gridrt::GridParams* h_params = nullptr;      // pinned mirror, then a word for BuildWork::sticky
     gridrt::BuildWork* d_work = nullptr;
     int32_t* d_offsets = nullptr;
     int64_t cell_cap = 0;
@@ -63,6 +65,10 @@ struct rtg_scene_s {
     int32_t k = 0;
     gridrt::GridParams hp{};   // host copy of the last successful build
 
+    // rtg_render's buffers: a pool of the scene's own, made by its first frame
+    // and destroyed with it, that keeps up to kRenderKeep bytes between frames
+    std::once_flag render_once;
+    cudaMemPool_t render_pool = nullptr;
     unsigned char* d_io = nullptr;
     int64_t io_cap = 0;
     // rtg_trace_frame_async: shadow-ray area + two output slots, copied back
