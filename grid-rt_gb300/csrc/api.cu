@@ -184,22 +184,17 @@ void host_resolve(GridParams& p, int32_t k, int64_t ntris, int64_t cell_cap) {
 
 namespace {
 
-// The status bits of every build since the last clear live in BuildWork.
-char* sticky_addr(rtg_scene s) { return reinterpret_cast<char*>(s->d_work) + offsetof(BuildWork, sticky); }
-uint32_t* host_sticky(rtg_scene s) { return reinterpret_cast<uint32_t*>(s->h_params + 1); }
-
-// Parameters and sticky bits with one wait: a second one, for the sticky word
-// alone, made a 500-triangle build 67 us instead of 52.
-rtg_status read_params(rtg_scene s) {
-    CUDA_TRY(cudaMemcpyAsync(host_sticky(s), sticky_addr(s), sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaMemcpyAsync(s->h_params, s->d_params, sizeof(GridParams), cudaMemcpyDeviceToHost, s->stream));
+// The last build's parameters, and the status bits of every build since the
+// last clear (work.sticky), into h_state.
+rtg_status read_state(rtg_scene s) {
+    CUDA_TRY(cudaMemcpyAsync(s->h_state, s->d_state, sizeof(BuildState), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return RTG_OK;
 }
 
 rtg_status clear_sticky(rtg_scene s) {
-    if (*host_sticky(s) == 0u) return RTG_OK;
-    CUDA_TRY(cudaMemsetAsync(sticky_addr(s), 0, sizeof(uint32_t), s->stream));
+    if (s->h_state->work.sticky == 0u) return RTG_OK;
+    CUDA_TRY(cudaMemsetAsync(&s->d_work->sticky, 0, sizeof(uint32_t), s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return RTG_OK;
 }
@@ -309,9 +304,12 @@ rtg_status rtg_scene_create(int device, void* stream, rtg_scene* out) {
     s->bitmap_words = words;
     rtg_status rc = RTG_OK;
     if (build_setup_attributes(words) != cudaSuccess) rc = fail(RTG_DEVICE_ERROR, "smem attribute");
-    if (rc == RTG_OK && cudaMalloc(&s->d_params, sizeof(GridParams)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "params");
-    if (rc == RTG_OK && cudaMallocHost(&s->h_params, sizeof(GridParams) + 16) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "pinned");
-    if (rc == RTG_OK && cudaMalloc(&s->d_work, sizeof(BuildWork)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "work");
+    if (rc == RTG_OK && cudaMalloc(&s->d_state, sizeof(BuildState)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "params");
+    if (rc == RTG_OK && cudaMallocHost(&s->h_state, sizeof(BuildState)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "pinned");
+    if (rc == RTG_OK) {
+        s->d_params = &s->d_state->params;
+        s->d_work = &s->d_state->work;
+    }
     if (rc == RTG_OK && cudaMalloc(&s->d_ctr, sizeof(TraceCounters)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "ctr");
     if (rc == RTG_OK && cudaMalloc(&s->d_ray_ctr, 8 * kRayCounters * sizeof(unsigned long long)) != cudaSuccess)
         rc = fail(RTG_NO_MEMORY, "ray counters");
@@ -359,9 +357,8 @@ rtg_status rtg_scene_destroy(rtg_scene s) {
     cudaFree(s->d_idx);
     cudaFree(s->d_tris);
     cudaFree(s->d_wald);
-    cudaFree(s->d_params);
-    if (s->h_params) cudaFreeHost(s->h_params);
-    cudaFree(s->d_work);
+    cudaFree(s->d_state);
+    if (s->h_state) cudaFreeHost(s->h_state);
     cudaFree(s->d_offsets);
     cudaFree(s->d_occ);
     cudaFree(s->d_ray_ctr);
@@ -538,15 +535,15 @@ rtg_status rtg_scene_build_check(rtg_scene s, void* stream) {
     rtg_status rc = set_device(s);
     if (rc) return rc;
     CUDA_TRY(cudaStreamSynchronize(pick(s, stream)));
-    rc = read_params(s);
+    rc = read_state(s);
     if (rc == RTG_OK) rc = clear_sticky(s);
     if (rc) return rc;
-    const uint32_t st = s->h_params->status | *host_sticky(s);
+    const uint32_t st = s->h_state->params.status | s->h_state->work.sticky;
     if (st & (ST_CELL_CAP | ST_REF_CAP | ST_SORT_CAP | ST_AMBIGUOUS))
         return fail(RTG_NO_MEMORY, "asynchronous build needs a synchronous rebuild (capacity or resolution)");
     if (st & ST_TOO_BIG) return fail(RTG_INVALID_PARAM, "grid exceeds the int32 index space");
     if (st & ST_BAD_RANGE) return fail(RTG_INVALID_GEOMETRY, "non-finite vertex or triangle outside the grid");
-    s->hp = *s->h_params;
+    s->hp = s->h_state->params;
     s->built = true;
     return RTG_OK;
 }
@@ -576,9 +573,9 @@ rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) {
     for (int attempt = 0; attempt < 6; ++attempt) {
         rc = enqueue_build(s, k, skip_bbox, s->stream);
         if (rc) return rc;
-        rc = read_params(s);
+        rc = read_state(s);
         if (rc) return rc;
-        GridParams p = *s->h_params;
+        GridParams p = s->h_state->params;
         if (p.status & ST_TOO_BIG) return fail(RTG_INVALID_PARAM, "grid exceeds the int32 index space");
         if (p.status & ST_AMBIGUOUS) {
             host_resolve(p, k, s->ntris, s->cell_cap);

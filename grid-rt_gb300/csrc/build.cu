@@ -1406,7 +1406,7 @@ static cudaError_t launch_cluster_k(void (*kernel)(KArgs...), unsigned grid, uns
 template <bool MULTI>
 static bool launch_build_impl(const BuildArgs& one, const BuildArgs* many, int ntasks, const BatchGrid& g,
                               bool skip_bbox, int bitmap_words, cudaStream_t st, const BuildFork* fork = nullptr) {
-    count_launches(9);
+    count_launches(7);
     const int* f[kBuildKinds];
     for (int k = 0; k < kBuildKinds; ++k) f[k] = MULTI ? g.first[k] : nullptr;
     // the triangle records: on the record stream beside the whole build (it
@@ -1443,21 +1443,33 @@ static bool launch_build_impl(const BuildArgs& one, const BuildArgs* many, int n
     launch_k(scan_reduce_kernel<MULTI>, g.total[BK_TILE], SCAN_THREADS, 0, st, one, many, f[BK_TILE], ntasks);
     launch_k(scan_down_kernel<MULTI>, g.total[BK_TILE], SCAN_THREADS, 0, st, one, many, f[BK_TILE], ntasks);
     launch_k(scatter_kernel<MULTI>, g.total[BK_TRI], 256, 0, st, one, many, f[BK_TRI], ntasks);
+    // a list holds a triangle once, so a scene of few triangles has no list for
+    // the longer sorts: their launches are left out (500 triangles: no cluster
+    // sort, 52 -> 48 us a synchronous build; 20: nor the other two, 40 -> 38)
+    const bool medium = MULTI || one.ntris > SORT_SMALL_MAX;
+    const bool large = MULTI || one.ntris > SORT_MED_MAX;
     // the three size classes sort disjoint cells: with side streams they run
-    // side by side, joined before the records pass reads the lists
+    // side by side, joined before the records pass reads the lists (500
+    // triangles: 26.6 us a build in a graph, 28.2 on one stream; 65,536: 822
+    // and 875)
     cudaStream_t sm = st, sl = st;
-    if (fork) {
+    if (fork && medium) {
         cudaEventRecord(fork->fork, st);
-        cudaStreamWaitEvent(fork->side[0], fork->fork, 0);
-        cudaStreamWaitEvent(fork->side[1], fork->fork, 0);
         sm = fork->side[0];
-        sl = fork->side[1];
+        cudaStreamWaitEvent(sm, fork->fork, 0);
+        if (large) {
+            sl = fork->side[1];
+            cudaStreamWaitEvent(sl, fork->fork, 0);
+        }
     }
     launch_k(sort_small_kernel<MULTI>, g.total[BK_SSMALL], 256, 0, st, one, many, f[BK_SSMALL], ntasks);
-    launch_k(sort_medium_kernel<MULTI>, g.total[BK_SMED], 512, 0, sm, one, many, f[BK_SMED], ntasks);
+    if (medium) {
+        count_launches(1);
+        launch_k(sort_medium_kernel<MULTI>, g.total[BK_SMED], 512, 0, sm, one, many, f[BK_SMED], ntasks);
+    }
     // a single-scene build whose ids fit one bitmap span sorts its lists
     // above kSplitRefs entries with a cluster each, first (the longest work)
-    bool split = !MULTI && one.ntris > 0 && one.ntris <= (int64_t)bitmap_words * 32;
+    bool split = !MULTI && one.ntris > kSplitRefs && one.ntris <= (int64_t)bitmap_words * 32;
     if (split) {
         const int clusters = one.num_sms / kSplitBlocks > 0 ? one.num_sms / kSplitBlocks : 1;
         const int64_t words = ((one.ntris + kSplitBlocks - 1) / kSplitBlocks + 31) / 32 + 1;
@@ -1471,12 +1483,17 @@ static bool launch_build_impl(const BuildArgs& one, const BuildArgs* many, int n
             split = false;
         }
     }
-    launch_k(sort_large_kernel<MULTI>, g.total[BK_SLARGE], 1024, (size_t)bitmap_words * 4, sl, one, many,
-             f[BK_SLARGE], ntasks, split);
-    if (fork) {
+    if (large) {
+        count_launches(1);
+        launch_k(sort_large_kernel<MULTI>, g.total[BK_SLARGE], 1024, (size_t)bitmap_words * 4, sl, one, many,
+                 f[BK_SLARGE], ntasks, split);
+    }
+    if (sm != st) {
         cudaEventRecord(fork->join[0], sm);
-        cudaEventRecord(fork->join[1], sl);
         cudaStreamWaitEvent(st, fork->join[0], 0);
+    }
+    if (sl != st) {
+        cudaEventRecord(fork->join[1], sl);
         cudaStreamWaitEvent(st, fork->join[1], 0);
     }
     if (rec_side) cudaStreamWaitEvent(st, fork->rec_join, 0);

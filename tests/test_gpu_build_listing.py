@@ -46,3 +46,25 @@ def test_listing(gridlib, oracle, name, k):
     assert s.build_check() == 0
     off, ids = s.download()
     assert np.array_equal(off, g.offsets) and np.array_equal(ids, g.ids)
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 32, 33, 256, 257, 4096, 4097])
+def test_longest_list_of_a_scene(gridlib, oracle, n):
+    """A list of as many entries as the scene has triangles, at the sizes where
+    the sorts of longer lists are no longer launched."""
+    rng = np.random.default_rng(n)
+    sc = _soup(rng, n, np.full(n, 0.2))
+    v = sc.verts.reshape(-1, 3, 3)
+    v[:] = v * 1e-4 + np.float32([0.21, 0.33, -0.27])
+    v[rng.integers(n)] = [[0.0, 0.0, 0.0], [1.0, 1.0, 0.5], [-1.0, -0.5, -1.0]]   # its range covers every cell
+    s = gridlib.Scene(0)
+    s.set_geometry(sc.verts, sc.idx)
+    g = oracle.Grid(sc.verts, sc.idx, 2)
+    assert np.diff(g.offsets).max() == n
+    s.build(2)
+    off, ids = s.download()
+    assert np.array_equal(off, g.offsets) and np.array_equal(ids, g.ids)
+    s.build_async(2)
+    assert s.build_check() == 0
+    off, ids = s.download()
+    assert np.array_equal(off, g.offsets) and np.array_equal(ids, g.ids)
