@@ -111,7 +111,7 @@ struct TraceTuning {
     int empty_run = 4;     // empty cells a lane may walk per loop iteration: 2, 4, 8 or 16
     int persistent = 1;    // 1: persistent warps over ray batches; 0: one batch per warp
     int cell_records = 0;  // 1: the build also writes triangle records in cell-list order
-    int heavy_cell = 32;   // > 0: rays meeting a list longer than this finish in a warp-per-ray pass
+    int heavy_cell = 32;   // > 0: rays meeting a list longer than this finish in a group-of-lanes pass
     int heavy_lanes = 32;  // lanes per deferred ray in that pass: 4, 8, 16 or 32
     int refill = -1;       // > 0: idle lanes take new rays once this many are idle (0: finish each batch of 32);
                            // -1 (default): 8 for rays given as arrays, off for camera and frame traces
@@ -137,12 +137,19 @@ inline int refill_for(const TraceTuning& t, int mode_is_camera) {
 // 252 / 188 / 169 / 222, 256,000 rays 336 / 356 / 333 / 427; frames (each ray
 // followed by its shadow ray, uneven over the image) of the same triangles:
 // 64,000 pixels 348 / 96 / 83 / 103, 256,000 376 / 189 / 231 / 357, 512,000
-// 423 / 327 / 438 / 702 -- but 512,000 pixels of the sphere 246 / 331.
-inline int lanes_for(long long n, int sms, int mode_is_camera) {
+// 423 / 327 / 438 / 702 -- but 512,000 pixels of the sphere 246 / 331.  Where
+// walks are short one ray a lane fills the GPU sooner, so `quarters` (of the
+// resident lanes: the most rays that get 8 lanes) is 4 for closest hits, 3 for
+// occlusion and 7 for frames: in 5,000 triangles, several launches in flight,
+// 155,000 closest-hit rays take 81 us at 8 lanes and at one, 155,000 occlusion
+// segments 120 and 101; frames at 8 lanes and one, 512 x 512: plane and debris
+// 178 and 333, the sphere 120 and 129; 300 x 1,000, the sphere filling the
+// image: 193 and 151.
+inline int lanes_for(long long n, int sms, int quarters) {
     const long long resident = 1024LL * sms;
     if (8 * n <= resident) return 32;
     if (2 * n <= resident) return 16;
-    return n <= (mode_is_camera ? 2 * resident : resident + resident / 4) ? 8 : 1;
+    return 4 * n <= quarters * resident ? 8 : 1;
 }
 
 // Kernel launch with programmatic stream serialisation when GRIDRT_PDL is on

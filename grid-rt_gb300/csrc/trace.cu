@@ -57,7 +57,7 @@ __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P
                 const int rank = __popc(idle & ((1u << lane) - 1u));
                 if (rank < take) {
                     L.ray = at + rank;
-                    set_deferral(L, io.heavy);
+                    set_deferral(L, io.heavy, io.work);
                     ++started;
                     if (start_ray<MODE_TASK>(P, io, L, L.ray)) {
                         active = true;
@@ -90,7 +90,7 @@ __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P
                                                    L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
                         active = false;
                     } else {
-                        set_deferral(L, kNoHeavy);
+                        set_deferral(L, kNoHeavy, kNoHeavy);
                         L.id = -1;
                     }
                     fin = false;
@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(128, GRIDRT_TRACE_MIN_BLOCKS)
         io.defer = defer;
         io.defer_cap = defer_cap;
         io.heavy = defer ? heavy : kNoHeavy;
+        io.work = work_limit(io.heavy, kHeavyWorkMult);
         io.defer_base = (int32_t)T.first;
         io.refill = refill;
         io.any = T.mode == MODE_ANY;
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(128, GRIDRT_INST_MIN_BLOCKS) trace_instances_k
                 xf_dir(m, wd[0], wd[1], wd[2], L.dx, L.dy, L.dz);
                 active = setup_ray(P, L, tn, tf);
                 L.tmax = tmax;
-                set_deferral(L, kNoHeavy);
+                set_deferral(L, kNoHeavy, kNoHeavy);
                 if (MODE == MODE_NEAREST) L.best = gbest;
             }
             const SceneView V = rec->view;
@@ -482,6 +483,7 @@ void launch_trace_instances(const InstanceRec* recs, void* d_params, int ninst, 
     io.counter = counter;
     io.ctr = ctr;
     io.heavy = kNoHeavy;
+    io.work = kNoHeavy;
     const int er = tune.empty_run;
     if (mode == MODE_ANY) {
         if (er <= 2) launch_instances_er<MODE_ANY, 2>(recs, sp, spheres, ninst, box, io, inst_out, tune, num_sms, st);
@@ -541,7 +543,7 @@ void launch_trace_batch(const BatchScene* scenes, int nscenes, const BatchTask* 
                         const TraceSlot& slot, const TraceTuning& tune, int num_sms, cudaStream_t st) {
     if (total <= 0 || ntasks <= 0) return;
     // deferred entries are int32 flattened indices
-    const int lanes = tune.lanes || total > 0x7fffffffLL ? 1 : lanes_for(total, num_sms, 0);
+    const int lanes = tune.lanes || total > 0x7fffffffLL ? 1 : lanes_for(total, num_sms, 4);
     if (lanes > 1) {
         // a small batch: every ray by a group of lanes, long lists dealt out
         // over it

@@ -22,10 +22,14 @@
 // rays to its idle lanes as it goes).  Per loop iteration a lane walks up to
 // ER empty cells (a tuning parameter), decided from a 4x4x2-brick occupancy
 // bitmap whose current word stays in a register, and tests at most one
-// non-empty cell, so lanes that reach triangles test them together.  A frame
+// non-empty cell (camera rays and coherent arrays: the whole list; other
+// arrays: two entries, so that lanes at short lists need not wait for the
+// longest), so lanes that reach triangles test them together.  A frame
 // (MODE_FRAME) traces each camera ray's shadow ray in the same lane right
 // after it.  Rays that meet a long list finish in a group-of-lanes pass,
 // those that then meet a dense cluster's list in a block-per-ray pass.
+// Launches too small to fill the GPU with one ray a lane (lanes_for) start in
+// groups of lanes, which walk consecutive cells of one ray side by side.
 #pragma once
 
 #include "common.cuh"
@@ -38,14 +42,11 @@ namespace gridrt {
 static constexpr float kChunkCells = 4.0f;   // chunk_coherent: origins, in cells
 static constexpr float kChunkCone = 0.1f;    // and directions, of the first ray's length
 static constexpr unsigned FULL = 0xffffffffu;
-static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the warp-per-ray pass
+static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the group-of-lanes pass
 static constexpr int32_t kNoHeavy = 0x7fffffff;
 // A ray is also deferred once its tests would pass kHeavyWorkMult x the
-// heavy-cell threshold in total (0: only long lists defer).
-#ifndef GRIDRT_HEAVY_WORK_MULT
-#define GRIDRT_HEAVY_WORK_MULT 8
-#endif
-static constexpr int32_t kHeavyWorkMult = GRIDRT_HEAVY_WORK_MULT;
+// heavy-cell threshold in total (frames: work_mult).
+static constexpr int32_t kHeavyWorkMult = 8;
 
 
 // MODE_FRAME: a camera ray, then in the same lane the shadow ray of its hit
@@ -96,7 +97,7 @@ struct Lane {
     int32_t cw;          // cached occupancy word index
     uint32_t cword;      // its value
     int32_t ray;         // ray index within the launch or task, -1 = none
-    int32_t li, le;      // entries of the current cell's list not yet tested (advance); li >= le: walking
+    int32_t li, le;      // entries of the current cell's list not yet tested (advance_two); li >= le: walking
     bool fast_best;      // best is Moller-Trumbore's t of an accepted entry (test_tri_fast)
 };
 
@@ -107,10 +108,14 @@ __device__ __forceinline__ bool any_hit_phase(const Lane& L) {
 }
 
 // When the one-lane walk hands the lane's ray on: at a list above `heavy`, or
-// once its tests would pass kHeavyWorkMult x heavy (kNoHeavy: never).
-__device__ __forceinline__ void set_deferral(Lane& L, int32_t heavy) {
+// once its tests would pass `work` (kNoHeavy: never).
+__device__ __forceinline__ void set_deferral(Lane& L, int32_t heavy, int32_t work) {
     L.heavy = heavy;
-    L.work = heavy < kNoHeavy / (kHeavyWorkMult + 1) && kHeavyWorkMult > 0 ? heavy * kHeavyWorkMult : kNoHeavy;
+    L.work = work;
+}
+
+inline __host__ __device__ int32_t work_limit(int32_t heavy, int32_t mult) {
+    return heavy < kNoHeavy / (mult + 1) ? heavy * mult : kNoHeavy;
 }
 
 // Ray::update + AabbIntersection::clipRay + traverse3ddda set-up
@@ -541,6 +546,7 @@ struct TraceIO {
     int2* defer;                   // deferred rays {ray index, cell it stopped at} (nullptr: no deferral)
     int32_t defer_cap;
     int32_t heavy;                 // lists longer than this are deferred (kNoHeavy: never)
+    int32_t work;                  // and rays with more tests than this
     int32_t defer_base;            // added to a deferred ray's index (a batch task's first)
     int32_t refill;                // > 0: lane refill at this many idle lanes (trace_refill)
     int any;                       // TASK: occlusion (else closest hits)
@@ -701,7 +707,7 @@ __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView&
     const long long ray = base + lane;
     bool active = ray < io.n;
     L.ray = (int32_t)ray;
-    set_deferral(L, io.heavy);
+    set_deferral(L, io.heavy, io.work);
     if (active) {
         ++started;
         if (!start_ray<MODE>(P, io, L, L.ray)) {
@@ -723,11 +729,11 @@ __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView&
                 if (d) {
                     const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
                     if (slot < (unsigned long long)io.defer_cap) {
-                        // the walk resumes at this cell in the warp-per-ray pass
+                        // the walk resumes at this cell in the group-of-lanes pass
                         io.defer[slot] = make_int2(defer_tag<MODE>(L, io), L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
                         active = false;
                     } else {
-                        set_deferral(L, kNoHeavy);   // queue full: the lane tests the cell itself
+                        set_deferral(L, kNoHeavy, kNoHeavy);   // queue full: the lane tests the cell itself
                         L.id = -1;
                     }
                     fin = false;
@@ -814,7 +820,7 @@ __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& 
                 const long long ray = (long long)b + __popc(idle & ((1u << lane) - 1u));
                 if (ray < io.n) {
                     L.ray = (int32_t)ray;
-                    set_deferral(L, io.heavy);
+                    set_deferral(L, io.heavy, io.work);
                     ++started;
                     if (start_ray<MODE>(P, io, L, L.ray)) {
                         active = true;
@@ -845,7 +851,7 @@ __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& 
                                                    L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
                         active = false;
                     } else {
-                        set_deferral(L, kNoHeavy);
+                        set_deferral(L, kNoHeavy, kNoHeavy);
                         L.id = -1;
                     }
                     fin = false;
@@ -1654,6 +1660,17 @@ inline void launch_huge(const SceneView& s, const TraceIO& io, int num_sms, cuda
     launch_k(trace_huge_kernel<MODE, COUNT>, (unsigned)(per_sm * num_sms), kHugeThreads, kStageBytes, st, s, io);
 }
 
+// The tests after which a camera ray (with its shadow ray in a frame) is handed
+// to a group of lanes, in heavy-cell thresholds: the fewer the shorter the tail
+// of a launch, but its queue is fixed, so larger launches hand on fewer of
+// their rays.  Frames of the sphere / of plane and debris, us at 8 -> here:
+// 518,400 pixels 166 -> 133 / 398 -> 367 (4), 1,048,576 207 -> 186 /
+// 526 -> 530 (5).  Ray arrays stay at 8 (4 M random rays 2,254 us, at 4 2,321).
+inline int32_t work_mult(long long n, int sms) {
+    const long long m = 2 + n / (2048LL * sms);
+    return (int32_t)(m < 4 ? 4 : (m > kHeavyWorkMult ? kHeavyWorkMult : m));
+}
+
 template <int MODE>
 inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, const TraceTuning& tune, int num_sms,
                         cudaStream_t st) {
@@ -1667,17 +1684,29 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
     io.huge = defer ? slot.huge : nullptr;
     io.huge_cap = io.huge ? slot.huge_cap : 0;
     cudaMemsetAsync(slot.ctr, 0, 8 * sizeof(unsigned long long), st);
-    const int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera));
+    io.work = work_limit(io.heavy, kHeavyWorkMult);
+    if (camera && io.heavy != kNoHeavy) {   // below 128 tests only where the caller's threshold says so
+        const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms));
+        io.work = less > few ? less : few;
+    }
+    const int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera ? 7 : MODE == MODE_ANY ? 3 : 4));
     if (lanes > 1) {
-        // every ray walked by a group of lanes from its start.  A list that
-        // would take its lanes more than heavy_cell / 2 turns is deferred;
-        // groups of 16 and 32 deal any list out themselves, as do all when
-        // the scene had no such list
-        if (io.heavy < kNoHeavy / 64) io.heavy = io.heavy * lanes / 2;
-        if (lanes >= 16 || (!tune.lanes && slot.longest <= io.heavy)) {
+        // every ray walked by a group of lanes from its start.  Groups of 16
+        // and 32 deal any list out themselves, as do groups of 8 when no list
+        // of the scene would take them more than heavy_cell / 2 turns.  Where
+        // there are longer ones, 8 lanes hand on the lists above heavy_cell,
+        // as one lane does; 2 and 4 lanes (set by the caller) those of more
+        // than heavy_cell / 2 turns.  A 512^2 frame of the sphere with crowded
+        // poles (102,720 triangles, k = 4), 8 lanes: 198 us with several frames
+        // in flight and 261 alone; handing on above heavy_cell * 4, 233 and
+        // 296; one lane a ray, 215 and 281.
+        const bool known = io.heavy < kNoHeavy / 64;
+        const int32_t deal = known ? io.heavy * lanes / 2 : io.heavy;
+        if (lanes >= 16 || (!tune.lanes && slot.longest <= deal)) {
             io.defer = nullptr;
             io.defer_cap = 0;
         }
+        if (tune.lanes) io.heavy = deal;
     }
     count_launches(1 + (io.defer ? 1 : 0) + (io.huge ? 1 : 0));
     switch (lanes) {

@@ -44,7 +44,7 @@ def test_ray_arrays_by_groups_equal_one_lane(gridlib, name):
         assert np.array_equal(got[1], want[1]), (name, n)
 
 
-@pytest.mark.parametrize("side", [(8, 8), (136, 136), (272, 272), (280, 288), (552, 560), (568, 560)])
+@pytest.mark.parametrize("side", [(8, 8), (136, 136), (272, 272), (280, 288), (512, 528), (520, 528), (552, 560), (568, 560)])
 def test_frames_by_groups_equal_one_lane(gridlib, side):
     import torch
     sc = scenes.deforming_sphere(3)
