@@ -3,9 +3,10 @@
 The space: cells per triangle k (when the caller lets it vary), ray tile
 order (scanline / Morton 8x8), empty-cell run length, persistent vs one-shot
 trace grid, threads per block of the one-lane trace launch, lanes per ray
-from the start (one, or a group of 2 or 4 for every ray), the list length
-above which a ray is finished by the warp-per-ray pass and that pass's lanes
-per ray, cell-ordered triangle records, lane refill.  Each candidate is timed
+from the start (one, or a group of 2 or 4 for every ray; a scene whose lanes
+were never set picks them by the launch's size, which no value here asks
+for), the list length above which a ray is finished by the group-of-lanes
+pass and that pass's lanes per ray, cell-ordered triangle records, lane refill.  Each candidate is timed
 with a caller-supplied measurement (CUDA events on the scene's stream).
 Spaces of up to `exhaustive_max` candidates are searched exhaustively; larger
 ones by coordinate descent -- from the first value of every dimension, each

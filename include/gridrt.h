@@ -488,7 +488,8 @@ rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, const rtg_req
  *                        (nearest, any, batches) and off for camera and frame traces, whose
  *                        lanes follow a camera ray with its shadow ray
  *   RTG_TUNE_BLOCK       threads per block of the one-lane trace launch: 64, 128 (default) or 256
- *                        (every block size keeps 64 registers a thread and 32 warps an SM)
+ *                        (camera and frame traces, and arrays at 256, keep 64 registers a thread
+ *                        and 32 warps an SM; arrays at 64 or 128 keep 72 and 28)
  *   RTG_TUNE_LANES       lanes that trace each ray from its start: 1 (one ray a lane, the long
  *                        lists handed on as above), 2 or 4 (every ray walked by a group of lanes,
  *                        each at another of its next cells; lists above heavy-cell x lanes / 2
