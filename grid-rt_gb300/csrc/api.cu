@@ -607,7 +607,10 @@ rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) {
         // a scene with crowded lists keeps their triangles' bounding spheres:
         // make room the first time, and build once more with them
         if (p.max_list > (uint32_t)kSplitRefs && s->csph_cap < ref_capacity(s) && attempt < 4) {
-            if (grow(s->d_csph, s->csph_cap, ref_capacity(s)) == cudaSuccess) continue;
+            if (grow(s->d_csph, s->csph_cap, ref_capacity(s)) == cudaSuccess) {
+                skip_bbox = false;   // the box pass clears the totals the next build adds into
+                continue;
+            }
             cudaGetLastError();   // without them the block-per-ray pass reads the records
         }
         s->hp = p;
