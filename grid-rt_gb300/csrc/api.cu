@@ -179,6 +179,7 @@ void host_resolve(GridParams& p, int32_t k, int64_t ntris, int64_t cell_cap) {
     p.ntris = ntris;
     p.status = st;
     p.max_list = 0u;
+    p.spheres = nullptr;
 }
 }  // namespace gridrt
 
@@ -203,7 +204,7 @@ rtg_status enqueue_build(rtg_scene s, int32_t k, bool skip_bbox, cudaStream_t st
     if (skip_bbox)
         CUDA_TRY(cudaMemsetAsync(reinterpret_cast<char*>(s->d_work) + offsetof(BuildWork, nsort), 0,
                                  sizeof(BuildWork::nsort), st));
-    s->csph_built = launch_build(make_args(s, k, skip_bbox), st, s->have_fork ? &s->fork : nullptr);
+    launch_build(make_args(s, k, skip_bbox), st, s->have_fork ? &s->fork : nullptr);
     CUDA_TRY(cudaGetLastError());
     return RTG_OK;
 }
@@ -254,7 +255,6 @@ SceneView scene_view(rtg_scene s) {
     v.ids = s->d_ids;
     v.occ = s->d_occ;
     v.crec = (s->tune.cell_records && s->crec_built) ? s->d_crec : nullptr;
-    v.csph = s->csph_built ? s->d_csph : nullptr;
     v.tris = s->d_tris;
     v.wald = s->d_wald;
     return v;
@@ -1096,7 +1096,6 @@ rtg_status rtg_batch_build_async(rtg_batch b, void* stream) {
         if (rc == RTG_OK) rc = apply_staged(sc, st);
         if (rc) return rc;
         sc->crec_built = sc->tune.cell_records != 0;   // this build writes them
-        sc->csph_built = false;                        // and no spheres (batch traces have no block-per-ray pass)
     }
     rtg_status rc = batch_upload_build(b, st, false);
     if (rc == RTG_OK) rc = batch_upload_views(b, st, false);

@@ -184,6 +184,7 @@ __device__ __forceinline__ void bbox_params_body(const float* __restrict__ verts
     p->ntris = ntris;
     p->status = status;
     p->max_list = 0u;
+    p->spheres = nullptr;
     if (status) atomicOr(&w->sticky, status);
 }
 
@@ -1190,6 +1191,7 @@ __device__ __forceinline__ float4 hit_sphere(const float4& A, const float4& B, c
 __global__ void __launch_bounds__(1024) sort_split_kernel(BuildArgs a) {
     pdl_begin();
     if (sort_skip(a.params)) return;
+    if (a.csph && blockIdx.x == 0 && threadIdx.x == 0) a.params->spheres = a.csph;   // the passes after this read them
     extern __shared__ uint32_t sbm[];
     __shared__ int32_t warp_tot[32];
     __shared__ int32_t slice_total;
@@ -1404,7 +1406,7 @@ static cudaError_t launch_cluster_k(void (*kernel)(KArgs...), unsigned grid, uns
 }
 
 template <bool MULTI>
-static bool launch_build_impl(const BuildArgs& one, const BuildArgs* many, int ntasks, const BatchGrid& g,
+static void launch_build_impl(const BuildArgs& one, const BuildArgs* many, int ntasks, const BatchGrid& g,
                               bool skip_bbox, int bitmap_words, cudaStream_t st, const BuildFork* fork = nullptr) {
     count_launches(7);
     const int* f[kBuildKinds];
@@ -1501,13 +1503,12 @@ static bool launch_build_impl(const BuildArgs& one, const BuildArgs* many, int n
         count_launches(1);
         launch_k(cell_records_kernel<MULTI>, g.total[BK_REFS], 256, 0, st, one, many, f[BK_REFS], ntasks);
     }
-    return split && one.csph;
 }
 
-bool launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork) {
+void launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork) {
     BatchGrid g{};
     build_blocks(a, a.num_sms, g.total);
-    return launch_build_impl<false>(a, nullptr, 1, g, a.skip_bbox, a.bitmap_words, st, fork);
+    launch_build_impl<false>(a, nullptr, 1, g, a.skip_bbox, a.bitmap_words, st, fork);
 }
 
 void launch_build_batch(const BuildArgs* d_tasks, int ntasks, const BatchGrid& g, int bitmap_words,

@@ -28,6 +28,11 @@ struct GridParams {
     int64_t ntris;
     uint32_t status;
     uint32_t max_list;    // longest cell list of the build (set by the scan)
+    // bounding spheres of the lists above kSplitRefs, in list order: cleared
+    // where a build's parameters are set, written by the sort that makes them,
+    // so a trace never reads those of other lists (a replayed graph changes the
+    // grid without a word to the host)
+    const float4* spheres;
 };
 
 // status bits written by the build kernels

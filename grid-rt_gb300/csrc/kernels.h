@@ -62,8 +62,7 @@ struct BuildFork {
     cudaEvent_t rec_clear;   // the offsets and bitmap cleared (the count pass waits for it)
     cudaEvent_t rec_join;
 };
-// True when the lists above kSplitRefs got their bounding spheres (a.csph).
-bool launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork = nullptr);
+void launch_build(const BuildArgs& a, cudaStream_t st, const BuildFork* fork = nullptr);
 
 // Build kernels by work shape (grid sizing per task).
 enum BuildKind { BK_BBOX = 0, BK_ZERO, BK_TRI, BK_TILE, BK_SSMALL, BK_SMED, BK_SLARGE, BK_REFS, BK_RECS, kBuildKinds };
@@ -91,7 +90,6 @@ struct SceneView {
     const int32_t* ids;
     const uint32_t* occ;
     const float4* crec;    // records in cell-list order, or nullptr (then ids -> tris)
-    const float4* csph;    // bounding spheres of the lists above kSplitRefs in list order, or nullptr
     const float4* tris;
     const float4* wald;    // TriAccel records: the reported t / u / v of a hit (nullptr: from tris)
 };

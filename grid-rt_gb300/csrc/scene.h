@@ -70,7 +70,6 @@ struct rtg_scene_s {
 
     bool built = false;
     bool crec_built = false;             // the last build wrote cell-ordered records
-    bool csph_built = false;             // the last build wrote the crowded lists' spheres
     int32_t k = 0;
     gridrt::GridParams hp{};   // host copy of the last successful build
 

@@ -1250,6 +1250,7 @@ struct Stage {
     int* off;             // shared: 1 once a wait has run out
     int32_t* cand;        // shared: candidates of a list's spheres, kCand at most
     int* cand_n;          // shared: how many there were
+    const float4* spheres;   // of the lists above kSplitRefs (GridParams::spheres), or nullptr
     uint32_t phase;       // bit q: the parity of buffer q's next completion
 };
 
@@ -1388,12 +1389,12 @@ __device__ __forceinline__ void block_walk(const SParams& P, const SceneView& s,
             // cluster) are queued in shared memory and tested together behind
             // the list's last chunk -- a warp that tested its own at once
             // waited for their loads at every step
-            const bool sph = s.csph && e - b > kSplitRefs;
+            const bool sph = st && st->spheres && e - b > kSplitRefs;
             const float grow = sph ? 256.0f * kRound * (o1 + 2.0f * cell_l1(P, c)) : 0.0f;
             if (GRIDRT_STAGE && st && (sph || (s.crec && e - b >= kStageMin)) && !*st->off) {
                 // staged: chunk ch in buffer ch % kStageDepth, the next
                 // kStageDepth - 1 chunks in flight
-                const float4* __restrict__ src = sph ? s.csph : s.crec;
+                const float4* __restrict__ src = sph ? st->spheres : s.crec;
                 const int32_t quads = sph ? 1 : 3, per = sph ? 3 * kStageEntries : kStageEntries;
                 const int32_t nch = (e - b + per - 1) / per;
                 if (sph) {
@@ -1544,7 +1545,7 @@ __global__ void __launch_bounds__(kHugeThreads, GRIDRT_HUGE_MIN_BLOCKS) trace_hu
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         stage_off = 0;
     }
-    Stage stage{stage_buf, stage_bar, &stage_off, cand, &cand_n, 0u};
+    Stage stage{stage_buf, stage_bar, &stage_off, cand, &cand_n, s.params->spheres, 0u};
     load_sparams(s.params, P);
     unsigned long long nh = io.counter[3];
     if (nh > (unsigned long long)io.huge_cap) nh = (unsigned long long)io.huge_cap;

@@ -41,3 +41,109 @@ def test_crowded_scene_of_host_resolved_parameters(gridlib, oracle):
         off, ids = s.download()
         assert np.array_equal(off, g.offsets) and np.array_equal(ids, g.ids)
     s.close()
+
+
+def _reversed_crowd(sc):
+    """The same triangles, the crowd's in the reverse order: the same lists, but
+    another triangle at every place of them."""
+    v = sc.verts.reshape(-1, 3, 3).copy()
+    v[60:] = v[60:][::-1]
+    return v.reshape(-1, 3)
+
+
+def _crowd_rays(sc, n=3000):
+    mid = sc.verts.reshape(-1, 3, 3)[60:].mean(axis=(0, 1))
+    rng = np.random.default_rng(n)
+    rays = scenes.random_rays(rng, n, mid - 4, mid + 4)
+    rays[:, 4:7] = (mid + rng.normal(size=(n, 3)) * 0.01 - rays[:, 0:3]).astype(np.float32)
+    return rays
+
+
+def _hits_of(gridlib, verts, idx, rays):
+    s = gridlib.Scene(0)
+    s.set_geometry(verts, idx)
+    s.build(1)
+    s.set_tuning(heavy_cell=0, lanes=2)      # every entry tested
+    hits = s.trace_nearest(rays).view(np.int32)
+    s.close()
+    return hits
+
+
+@pytest.fixture()
+def moved(gridlib):
+    sc = _crowd("tiny", 9000)
+    rays = _crowd_rays(sc)
+    verts = _reversed_crowd(sc)
+    before, after = _hits_of(gridlib, sc.verts, sc.idx, rays), _hits_of(gridlib, verts, sc.idx, rays)
+    assert (before[:, 0] != after[:, 0]).mean() > 0.2
+    return sc, verts, rays, before, after
+
+
+def _capture(stream, call):
+    import torch
+    call()                                   # tables and modules before the capture
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        call()
+    return g
+
+
+def test_replayed_batch_build_of_a_scene_with_spheres(gridlib, moved):
+    """A captured batch rebuilds a scene whose own build had written spheres."""
+    import torch
+    sc, verts, rays, before, after = moved
+    s = gridlib.Scene(0)
+    s.set_geometry(sc.verts, sc.idx)
+    out = torch.zeros((64, 4), dtype=torch.int32, device="cuda")
+    b = gridlib.Batch([s], [1], [(0, gridlib.RTG_MODE_NEAREST, torch.from_numpy(rays[:64]).cuda(), 64, out)])
+    stream = torch.cuda.Stream()
+
+    def step():
+        b.build_async(stream.cuda_stream)
+        b.trace_async(stream.cuda_stream)
+
+    g = _capture(stream, step)
+    s.build(1)
+    assert np.array_equal(s.trace_nearest(rays).view(np.int32), before)
+    s.update_vertices(verts, len(verts), False)
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    assert b.check() == 0
+    assert np.array_equal(out.cpu().numpy(), after[:64])
+    assert np.array_equal(s.trace_nearest(rays).view(np.int32), after)
+
+
+def test_replayed_trace_of_a_scene_a_batch_rebuilt(gridlib, moved):
+    """A captured trace of a scene with spheres, after a batch has rebuilt it;
+    and again once its own build has written them anew."""
+    import torch
+    sc, verts, rays, before, after = moved
+    s = gridlib.Scene(0)
+    s.set_geometry(sc.verts, sc.idx)
+    b = gridlib.Batch([s], [1], [])
+    s.build(1)
+    d_rays, hits = torch.from_numpy(rays).cuda(), torch.zeros((len(rays), 4), dtype=torch.int32, device="cuda")
+    stream = torch.cuda.Stream()
+    g = _capture(stream, lambda: s.trace_nearest_device(d_rays, len(rays), hits, stream=stream.cuda_stream))
+
+    def replay():
+        hits.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        return hits.cpu().numpy()
+
+    assert np.array_equal(replay(), before)
+    s.update_vertices(verts, len(verts), False)
+    torch.cuda.synchronize()
+    b.build_async()
+    assert b.check() == 0
+    assert np.array_equal(replay(), after)
+    s.build(1)
+    assert np.array_equal(replay(), after)
+    s.update_vertices(sc.verts, len(sc.verts), False)
+    s.build_async(1)
+    torch.cuda.synchronize()
+    assert np.array_equal(replay(), before)
