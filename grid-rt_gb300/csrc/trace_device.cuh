@@ -101,10 +101,10 @@ struct Lane {
     bool fast_best;      // best is Moller-Trumbore's t of an accepted entry (test_tri_fast)
 };
 
-// Whether the lane's ray looks for occlusion before L.tmax.
+// Whether the lane's ray looks for occlusion before L.tmax (which may be NaN).
 template <int MODE>
 __device__ __forceinline__ bool any_hit_phase(const Lane& L) {
-    return MODE == MODE_ANY || ((MODE == MODE_FRAME || MODE == MODE_TASK) && L.tmax > -kFltMax);
+    return MODE == MODE_ANY || ((MODE == MODE_FRAME || MODE == MODE_TASK) && L.tmax != -INFINITY);
 }
 
 // When the one-lane walk hands the lane's ray on: at a list above `heavy`, or
