@@ -1390,7 +1390,9 @@ __device__ __forceinline__ void block_walk(const SParams& P, const SceneView& s,
             // the list's last chunk -- a warp that tested its own at once
             // waited for their loads at every step
             const bool sph = st && st->spheres && e - b > kSplitRefs;
-            const float grow = sph ? 256.0f * kRound * (o1 + 2.0f * cell_l1(P, c)) : 0.0f;
+            // (directions below 1e-10, whose squared distances round to too few
+            // bits, meet every sphere)
+            const float grow = !sph ? 0.0f : (dd >= 1e-20f ? 256.0f * kRound * (o1 + 2.0f * cell_l1(P, c)) : INFINITY);
             if (GRIDRT_STAGE && st && (sph || (s.crec && e - b >= kStageMin)) && !*st->off) {
                 // staged: chunk ch in buffer ch % kStageDepth, the next
                 // kStageDepth - 1 chunks in flight

@@ -1,0 +1,46 @@
+"""Rays whose directions are so short that their squares leave the float range's
+normal numbers: nothing they hit is passed over by a bounding sphere."""
+import numpy as np
+import pytest
+
+from gridrt import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _at_rim(rng, n, radius):
+    """Rays from distance 1 that pass the origin at almost `radius`."""
+    o = rng.normal(size=(n, 3))
+    o /= np.linalg.norm(o, axis=1, keepdims=True)
+    p = np.cross(o, rng.normal(size=(n, 3)))
+    p *= radius * rng.uniform(0.9, 0.9997, size=(n, 1)) / np.linalg.norm(p, axis=1, keepdims=True)
+    rays = scenes.random_rays(rng, n, (-1, -1, -1), (1, 1, 1))
+    rays[:, 0:3] = o
+    rays[:, 4:7] = p - o
+    return rays
+
+
+@pytest.mark.parametrize("log2", [-60, -70, -71.5, -72, -72.5, -73])
+def test_crowded_list_of_short_rays(gridlib, log2):
+    """9,000 triangles about one point, hit near their corners: at the rim of
+    their spheres."""
+    rng = np.random.default_rng(4)
+    q, _ = np.linalg.qr(rng.normal(size=(9000, 3, 3)))
+    a = 2 * np.pi * np.arange(3) / 3
+    star = np.einsum("nij,kj->nki", q, 0.3 * np.stack([np.cos(a), np.sin(a), 0 * a], 1))
+    star += rng.uniform(-2e-3, 2e-3, size=(9000, 1, 3))
+    box = rng.uniform(-4, 4, size=(60, 1, 3)) + rng.uniform(-0.3, 0.3, size=(60, 3, 3))
+    verts = np.concatenate([box, star]).astype(np.float32).reshape(-1, 3)
+    s = gridlib.Scene(0)
+    s.set_geometry(verts, np.arange(len(verts), dtype=np.int32).reshape(-1, 3))
+    s.build(1)
+    off, _ = s.download()
+    assert np.diff(off).max() > 4096
+    rays = _at_rim(rng, 20_000, 0.3)
+    rays[:, 4:7] *= np.float32(2.0 ** log2)
+    s.set_tuning(heavy_cell=0, lanes=2)      # every entry tested
+    want = s.trace_nearest(rays).view(np.int32)
+    assert (want[:, 0] >= 0).mean() > 0.9
+    s.set_tuning(heavy_cell=32, lanes=4)
+    assert np.array_equal(s.trace_nearest(rays).view(np.int32), want)
+    s.close()
