@@ -377,8 +377,10 @@ __global__ void __launch_bounds__(128, GRIDRT_INST_MIN_BLOCKS) trace_instances_k
             const float q2 = qx * qx + qy * qy + qz * qz, along = qx * wd[0] + qy * wd[1] + qz * wd[2];
             const float R2 = 1.02f * (R * R) + 1e-9f * q2, lim = R2 * dd;
             const float past = along - 1.001f * fminf(gbest, tf) * dd;     // beyond the best hit and the far clip
-            const bool cull = xx * xx + xy * xy + xz * xz > lim || (tn >= 0.0f && along < 0.0f && q2 > R2) ||
-                              (tn >= 0.0f && past > 0.0f && past * past > lim);
+            // (products below the normal floats round to too few bits to tell)
+            const bool tell = dd >= 1e-20f && R2 >= 1e-18f;
+            const bool cull = tell && (xx * xx + xy * xy + xz * xz > lim || (tn >= 0.0f && along < 0.0f && q2 > R2) ||
+                                       (tn >= 0.0f && past > 0.0f && past * past > lim));
             if (!__any_sync(FULL, alive && !cull)) continue;
             __syncwarp();
             {
