@@ -60,8 +60,11 @@ rtg_status set_device(rtg_scene s) {
     return RTG_OK;
 }
 
+// References the id buffers hold, and a build of the scene.
+int64_t id_capacity(const rtg_scene s) { return s->ids_cap < s->scratch_cap ? s->ids_cap : s->scratch_cap; }
+
 int64_t ref_capacity(const rtg_scene s) {
-    int64_t c = s->ids_cap < s->scratch_cap ? s->ids_cap : s->scratch_cap;
+    int64_t c = id_capacity(s);
     if (s->tune.cell_records) c = c < s->crec_cap / 3 ? c : s->crec_cap / 3;
     return c;
 }
@@ -84,7 +87,7 @@ rtg_status ensure_grid_buffers(rtg_scene s, int64_t cells_plus_one, int64_t refs
 // Cell-ordered records enabled after the id buffers were sized: give the
 // record buffer the same capacity before the next build.
 rtg_status ensure_cell_records(rtg_scene s) {
-    const int64_t raw = s->ids_cap < s->scratch_cap ? s->ids_cap : s->scratch_cap;
+    const int64_t raw = id_capacity(s);
     if (!s->tune.cell_records || !s->d_offsets || s->crec_cap >= 3 * raw) return RTG_OK;
     return ensure_grid_buffers(s, s->cell_cap, raw);
 }
@@ -548,7 +551,27 @@ rtg_status rtg_scene_build_check(rtg_scene s, void* stream) {
     return RTG_OK;
 }
 
-rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) {
+// Makes room for the bounding spheres of a scene's crowded lists, as many as
+// the id buffers hold, so that a graph's builds and traces keep the buffer for
+// as long as they keep those.  True when it was too small before.
+static bool grow_spheres(rtg_scene s) {
+    const int64_t n = id_capacity(s);
+    if (s->csph_cap >= n) return false;
+    cudaFree(s->d_csph);   // the build just read did not fit it: the grid names no spheres
+    s->d_csph = nullptr;
+    s->csph_cap = 0;
+    if (cudaMalloc(&s->d_csph, (size_t)n * sizeof(float4)) != cudaSuccess) {
+        cudaGetLastError();   // without them the block-per-ray pass reads the records
+        s->d_csph = nullptr;
+        return false;
+    }
+    s->csph_cap = n;
+    return true;
+}
+
+// `spheres`: whether crowded lists may get their bounding spheres (the builds of
+// a batch write none).
+static rtg_status build_now(rtg_scene s, int32_t k, void* stream, bool spheres) {
     if (!s) return fail(RTG_INVALID_PARAM, "scene is NULL");
     if (k <= 0) return fail(RTG_INVALID_PARAM, "k must be positive");
     rtg_status rc = set_device(s);
@@ -606,12 +629,10 @@ rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) {
             return fail(RTG_INVALID_GEOMETRY, "non-finite vertex or triangle outside the grid");
         // a scene with crowded lists keeps their triangles' bounding spheres:
         // make room the first time, and build once more with them
-        if (p.max_list > (uint32_t)kSplitRefs && s->csph_cap < ref_capacity(s) && attempt < 4) {
-            if (grow(s->d_csph, s->csph_cap, ref_capacity(s)) == cudaSuccess) {
-                skip_bbox = false;   // the box pass clears the totals the next build adds into
-                continue;
-            }
-            cudaGetLastError();   // without them the block-per-ray pass reads the records
+        if (spheres && p.max_list > (uint32_t)kSplitRefs && sorts_split(s->ntris, s->bitmap_words) && attempt < 4 &&
+            s->csph_cap < ref_capacity(s) && grow_spheres(s)) {
+            skip_bbox = false;   // the box pass clears the totals the next build adds into
+            continue;
         }
         s->hp = p;
         s->built = true;
@@ -621,6 +642,8 @@ rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) {
     }
     return fail(RTG_DEVICE_ERROR, "grid build did not converge");
 }
+
+rtg_status rtg_scene_build(rtg_scene s, int32_t k, void* stream) { return build_now(s, k, stream, true); }
 
 rtg_status rtg_scene_grid_info(rtg_scene s, rtg_grid_info* out) {
     if (!s || !out) return fail(RTG_INVALID_PARAM, "NULL argument");
@@ -1039,7 +1062,7 @@ rtg_status rtg_batch_create(const rtg_scene* scenes, int32_t nscenes, const int3
     }
     CUDA_TRY(cudaSetDevice(dev));
     for (int i = 0; i < nscenes; ++i) {   // size every scene's buffers for its grid
-        rtg_status rc = rtg_scene_build(scenes[i], k[i], nullptr);
+        rtg_status rc = build_now(scenes[i], k[i], nullptr, false);
         if (rc) return rc;
     }
     rtg_batch b = new rtg_batch_s();

@@ -1471,7 +1471,7 @@ static void launch_build_impl(const BuildArgs& one, const BuildArgs* many, int n
     }
     // a single-scene build whose ids fit one bitmap span sorts its lists
     // above kSplitRefs entries with a cluster each, first (the longest work)
-    bool split = !MULTI && one.ntris > kSplitRefs && one.ntris <= (int64_t)bitmap_words * 32;
+    bool split = !MULTI && sorts_split(one.ntris, bitmap_words);
     if (split) {
         const int clusters = one.num_sms / kSplitBlocks > 0 ? one.num_sms / kSplitBlocks : 1;
         const int64_t words = ((one.ntris + kSplitBlocks - 1) / kSplitBlocks + 31) / 32 + 1;

@@ -41,6 +41,9 @@ struct BuildArgs {
 // bitmap span are sorted by sort_split_kernel, which also writes their
 // triangles' bounding spheres; the rest by sort_large.
 static constexpr int32_t kSplitRefs = SORT_BLOCK_MAX;
+inline bool sorts_split(int64_t ntris, int bitmap_words) {
+    return ntris > kSplitRefs && ntris <= (int64_t)bitmap_words * 32;
+}
 
 // Cells per tile of the count scan (tile sums: cell capacity / kScanTile + 2).
 static constexpr int kScanTile = 1024;

@@ -147,3 +147,46 @@ def test_replayed_trace_of_a_scene_a_batch_rebuilt(gridlib, moved):
     s.build_async(1)
     torch.cuda.synchronize()
     assert np.array_equal(replay(), before)
+
+
+def _launches(gridlib, call):
+    before = gridlib.kernel_launches()
+    call()
+    return gridlib.kernel_launches() - before
+
+
+def _reserved(gridlib, verts, idx, k):
+    """A scene with room for its grid, so that its first build needs no retry."""
+    s = gridlib.Scene(0)
+    s.set_geometry(verts, idx)
+    s.build(k)
+    info = s.info()
+    s.close()
+    s = gridlib.Scene(0)
+    s.set_geometry(verts, idx)
+    s.reserve(info["ncells"], info["nrefs"])
+    return s
+
+
+def test_no_spheres_where_no_build_writes_them(gridlib):
+    """A crowded scene of more ids than the cluster sort's bitmap span, and a
+    batch's sizing builds: one build each, none for spheres."""
+    rng = np.random.default_rng(8)
+    n = (1 << 20) + 1
+    v = rng.uniform(-1, 1, size=(n, 1, 3)) + rng.uniform(-0.004, 0.004, size=(n, 3, 3))
+    v[:6000] = rng.uniform(-1e-3, 1e-3, size=(6000, 3, 3)) + np.array([0.3, 0.2, 0.1])
+    s = _reserved(gridlib, v.astype(np.float32).reshape(-1, 3), np.arange(3 * n, dtype=np.int32).reshape(-1, 3), 1)
+    first, again = _launches(gridlib, lambda: s.build(1)), _launches(gridlib, lambda: s.build(1))
+    off, _ = s.download()
+    assert np.diff(off).max() > 4096 and first == again
+    s.close()
+
+    sc = _crowd("tiny", 9000)
+    s = _reserved(gridlib, sc.verts, sc.idx, 1)
+    batch = []
+    sizing = _launches(gridlib, lambda: batch.append(gridlib.Batch([s], [1], [])))
+    own = _launches(gridlib, lambda: s.build(1))          # now with spheres: two builds
+    assert 2 * sizing == own
+    assert _launches(gridlib, lambda: s.build(1)) == sizing
+    batch[0].close()
+    s.close()
