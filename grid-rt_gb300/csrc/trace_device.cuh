@@ -39,7 +39,7 @@
 
 namespace gridrt {
 
-static constexpr float kChunkCells = 4.0f;   // chunk_coherent: origins, in cells
+static constexpr float kChunkCells = 4.0f;   // chunk_alike: origins, in cells
 static constexpr float kChunkCone = 0.1f;    // and directions, of the first ray's length
 static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the group-of-lanes pass
@@ -770,25 +770,33 @@ constexpr int trace_min_blocks(int mode, int tpb) {
     return (mode == MODE_NEAREST || mode == MODE_ANY) && tpb <= 128 ? 7 * 128 / tpb : GRIDRT_TRACE_MIN_BLOCKS * 128 / tpb;
 }
 
-// Whether the 32 rays from `base` walk alike: origins within a few cells of the
-// first ray's and directions within a narrow cone of its (camera rays, shadow
-// rays of one surface).  Slots without a shadow ray (tfar < 0) count as alike.
+// Whether the 32 rays from `base` walk alike: of those that follow another ray,
+// 7 in 8 start within a few cells of it and go within a narrow cone of the first
+// ray's direction (camera rays, shadow rays of one surface or two).  Slots
+// without a shadow ray (tfar < 0) are neither.  1024^2 shadow rays of the sphere
+// and of plane and debris, scanline, 135 and 227 us; every origin against the
+// first slot's, which may hold no ray, 178 and 222; half of the pairs 135 and
+// 258.  Two cells: the sphere's 640 x 480 in Morton order 95 -> 119; a cone of
+// 0.05: its camera rays 192 -> 235; of 0.15, or of each ray's predecessor: 64
+// scenes in one batch, images of 50 to 400 pixels a row, 2,514 -> 2,539 and 2,565.
 // One component at a time: the lanes' walks are live around it.
 static __device__ __noinline__ bool chunk_alike(float cx, float cy, float cz, const float4* rays, int32_t n, int32_t base) {
     const int32_t r = min(base + (int32_t)(threadIdx.x & 31), n - 1);
     const float* __restrict__ q = reinterpret_cast<const float*>(rays + 2 * (int64_t)r);
     const float cell[3] = {cx, cy, cz};
+    const unsigned live = __ballot_sync(FULL, !(__ldg(q + 7) < 0.0f)), pairs = live & (live << 1);
+    const int first = live ? __ffs(live) - 1 : 0;
     bool alike = true;
     float off = 0.0f, len = 0.0f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float o = __ldg(q + a), d = __ldg(q + 4 + a);
-        const float o0 = __shfl_sync(FULL, o, 0), d0 = __shfl_sync(FULL, d, 0);
+        const float o0 = __shfl_up_sync(FULL, o, 1), d0 = __shfl_sync(FULL, d, first);
         if (!(fabsf(o - o0) <= kChunkCells * cell[a])) alike = false;
         off += fabsf(d - d0);
         len += fabsf(d0);
     }
-    return __all_sync(FULL, (alike && off <= kChunkCone * len) || __ldg(q + 7) < 0.0f);
+    return 8 * __popc(__ballot_sync(FULL, alike && off <= kChunkCone * len) & pairs) >= 7 * __popc(pairs);
 }
 __device__ __forceinline__ bool chunk_coherent(const SParams& P, const TraceIO& io, int32_t base) {
     return chunk_alike(P.cell[0], P.cell[1], P.cell[2], io.rays, (int32_t)io.n, base);
