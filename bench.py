@@ -1135,7 +1135,7 @@ def run_skewed(args, rank, ws, local, dist):
     else:
         space = {"k": LAMBDAS, "order": ("scanline", "morton8"), "empty_run": (2, 4, 8), "persistent": (True,),
                  "heavy_cell": (0, 24, 48), "heavy_lanes": (16, 32), "cell_records": (False, True),
-                 "refill": (0, 16), "block": (128, 64, 256), "lanes": (1, 2)}
+                 "refill": (0, 8, 16), "block": (128, 64, 256), "lanes": (-1, 1, 2)}
         best, allres = autotune.search(measure, space=space, reps=2)
         _save_autotune("skewed", allres)
     _apply_tuning(s, best)
@@ -1473,7 +1473,7 @@ def run_render(args, rank, ws, local, dist):
         s.render(cam, d_n, mats, lights, d_rgb, d_colors=d_c, d_material=d_m, max_depth=3)
         return 1e3 * (time.perf_counter() - t0)
 
-    best, allres = autotune.search(measure, space={"lanes": (1, 2, 4)}, reps=3)
+    best, allres = autotune.search(measure, space={"lanes": (-1, 1, 2, 4)}, reps=3)
     _save_autotune("render", allres)
     s.set_tuning(lanes=best["lanes"])
     for _ in range(args.warmup):

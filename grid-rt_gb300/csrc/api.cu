@@ -1246,9 +1246,9 @@ rtg_status rtg_scene_set_tuning(rtg_scene s, int32_t key, int32_t value) {
             s->tune.block = value;
             return RTG_OK;
         case RTG_TUNE_LANES:
-            if (value != 1 && value != 2 && value != 4)
-                return fail(RTG_INVALID_PARAM, "lanes per ray must be 1, 2 or 4");
-            s->tune.lanes = value;
+            if (value != -1 && value != 1 && value != 2 && value != 4)
+                return fail(RTG_INVALID_PARAM, "lanes per ray must be -1 (by the launch's size), 1, 2 or 4");
+            s->tune.lanes = value < 0 ? 0 : value;
             return RTG_OK;
         default:
             return fail(RTG_INVALID_PARAM, "unknown tuning key");

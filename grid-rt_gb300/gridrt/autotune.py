@@ -3,9 +3,8 @@
 The space: cells per triangle k (when the caller lets it vary), ray tile
 order (scanline / Morton 8x8), empty-cell run length, persistent vs one-shot
 trace grid, threads per block of the one-lane trace launch, lanes per ray
-from the start (one, or a group of 2 or 4 for every ray; a scene whose lanes
-were never set picks them by the launch's size, which no value here asks
-for), the list length above which a ray is finished by the group-of-lanes
+from the start (-1: by the launch's size, 1, or a group of 2 or 4 for every
+ray), the list length above which a ray is finished by the group-of-lanes
 pass and that pass's lanes per ray, cell-ordered triangle records, lane refill.  Each candidate is timed
 with a caller-supplied measurement (CUDA events on the scene's stream).
 Spaces of up to `exhaustive_max` candidates are searched exhaustively; larger
@@ -14,7 +13,8 @@ dimension in turn is set to its best value with the others fixed, until a
 full sweep changes nothing (at most `sweeps` sweeps) -- which times a few
 dozen candidates instead of every product.  The winner can be cached in a
 JSON file keyed by a workload signature, so a second run of the same
-workload skips the search; the result says whether it came from the cache.
+workload skips the search as long as the space is the same; the result says
+whether it came from the cache.
 None of these parameters changes a result: the grid and the hits are
 identical for every choice except k, which defines the grid.
 """
@@ -33,11 +33,11 @@ SPACE = {
     "empty_run": (4, 2, 8),
     "persistent": (True, False),
     "block": (128, 64, 256),
-    "lanes": (1, 2, 4),
+    "lanes": (-1, 1, 2, 4),
     "heavy_cell": (32, 0, 24, 48),
     "heavy_lanes": (32, 16),
     "cell_records": (False, True),
-    "refill": (0, 16),
+    "refill": (0, 8, 16),
 }
 
 
@@ -77,7 +77,8 @@ def search(measure: Callable[[dict], float], space: Dict[str, Iterable] = None, 
     or "search" for the last call."""
     space = {n: tuple(v) for n, v in (space or SPACE).items()}
     cache = _load() if (use_cache and key) else {}
-    if key and key in cache:
+    text = json.dumps(space, sort_keys=True)
+    if key and key in cache and cache[key].get("space") == text:
         search.last_source = "cache"
         return cache[key]["best"], [(c["cfg"], c["ms"]) for c in cache[key]["all"]]
     search.last_source = "search"
@@ -114,7 +115,8 @@ def search(measure: Callable[[dict], float], space: Dict[str, Iterable] = None, 
                 break
     if key:
         cache = _load()
-        cache[key] = {"best": best, "all": [{"cfg": c, "ms": m} for c, m in results], "when": time.time()}
+        cache[key] = {"best": best, "space": text, "all": [{"cfg": c, "ms": m} for c, m in results],
+                      "when": time.time()}
         _store(cache)
     return best, results
 

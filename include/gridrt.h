@@ -493,10 +493,10 @@ rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, const rtg_req
  *   RTG_TUNE_LANES       lanes that trace each ray from its start: 1 (one ray a lane, the long
  *                        lists handed on as above), 2 or 4 (every ray walked by a group of lanes,
  *                        each at another of its next cells; lists above heavy-cell x lanes / 2
- *                        handed on).  Unset, launches too small to fill the GPU with one ray a
- *                        lane use groups of 32, 16 or 8 lanes by their size and larger ones one
- *                        lane (65,536 triangles, 512^2 camera rays + their shadow rays, build
- *                        included: 0.47 ms at 1 lane, 0.32 at 2, 0.24 unset; 1024^2 frames:
+ *                        handed on).  -1 (default): launches too small to fill the GPU with one
+ *                        ray a lane use groups of 32, 16 or 8 lanes by their size and larger ones
+ *                        one lane (65,536 triangles, 512^2 camera rays + their shadow rays, build
+ *                        included: 0.47 ms at 1 lane, 0.32 at 2, 0.24 at -1; 1024^2 frames:
  *                        0.38 ms at 1, 0.55 at 2 or 4) */
 enum {
     RTG_TUNE_EMPTY_RUN = 1,
