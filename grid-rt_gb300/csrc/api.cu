@@ -44,7 +44,7 @@ cudaError_t grow(T*& p, int64_t& cap, int64_t need) {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc((void**)&p, (size_t)n * sizeof(T));
+    cudaError_t e = device_malloc(&p, (size_t)n * sizeof(T));
     if (e == cudaSuccess) cap = n;
     return e;
 }
@@ -70,17 +70,32 @@ int64_t ref_capacity(const rtg_scene s) {
 }
 
 
-rtg_status ensure_grid_buffers(rtg_scene s, int64_t cells_plus_one, int64_t refs) {
-    CUDA_TRY(grow(s->d_offsets, s->cell_cap, cells_plus_one));
-    CUDA_TRY(grow(s->d_occ, s->occ_cap, s->cell_cap));
-    CUDA_TRY(grow(s->d_tiles, s->tiles_cap, s->cell_cap / kScanTile + 2));
-    CUDA_TRY(grow(s->d_ids, s->ids_cap, refs));
-    CUDA_TRY(grow(s->d_scratch, s->scratch_cap, refs));
-    if (s->tune.cell_records) CUDA_TRY(grow(s->d_crec, s->crec_cap, 3 * s->ids_cap));
+cudaError_t grow_grid_buffers(rtg_scene s, int64_t cells_plus_one, int64_t refs) {
+    cudaError_t e = grow(s->d_offsets, s->cell_cap, cells_plus_one);
+    if (e == cudaSuccess) e = grow(s->d_occ, s->occ_cap, s->cell_cap);
+    if (e == cudaSuccess) e = grow(s->d_tiles, s->tiles_cap, s->cell_cap / kScanTile + 2);
+    if (e == cudaSuccess) e = grow(s->d_ids, s->ids_cap, refs);
+    if (e == cudaSuccess) e = grow(s->d_scratch, s->scratch_cap, refs);
+    if (e == cudaSuccess && s->tune.cell_records) e = grow(s->d_crec, s->crec_cap, 3 * s->ids_cap);
     const int64_t R = ref_capacity(s);
-    CUDA_TRY(grow(s->d_qs, s->qs_cap, R / 2 + 2));
-    CUDA_TRY(grow(s->d_qm, s->qm_cap, R / 33 + 2));
-    CUDA_TRY(grow(s->d_ql, s->ql_cap, R / (SORT_MED_MAX + 1) + 2));
+    if (e == cudaSuccess) e = grow(s->d_qs, s->qs_cap, R / 2 + 2);
+    if (e == cudaSuccess) e = grow(s->d_qm, s->qm_cap, R / 33 + 2);
+    if (e == cudaSuccess) e = grow(s->d_ql, s->ql_cap, R / (SORT_MED_MAX + 1) + 2);
+    return e;
+}
+
+rtg_status ensure_grid_buffers(rtg_scene s, int64_t cells_plus_one, int64_t refs) {
+    cudaError_t e = grow_grid_buffers(s, cells_plus_one, refs);
+    if (e == cudaErrorMemoryAllocation && s->d_csph) {
+        // the spheres only save time: their room is given up first
+        cudaGetLastError();
+        CUDA_TRY(cudaMemset(&s->d_params->spheres, 0, sizeof(float4*)));
+        cudaFree(s->d_csph);
+        s->d_csph = nullptr;
+        s->csph_cap = 0;
+        e = grow_grid_buffers(s, cells_plus_one, refs);
+    }
+    CUDA_TRY(e);
     return RTG_OK;
 }
 
@@ -307,17 +322,17 @@ rtg_status rtg_scene_create(int device, void* stream, rtg_scene* out) {
     s->bitmap_words = words;
     rtg_status rc = RTG_OK;
     if (build_setup_attributes(words) != cudaSuccess) rc = fail(RTG_DEVICE_ERROR, "smem attribute");
-    if (rc == RTG_OK && cudaMalloc(&s->d_state, sizeof(BuildState)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "params");
+    if (rc == RTG_OK && device_malloc(&s->d_state, sizeof(BuildState)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "params");
     if (rc == RTG_OK && cudaMallocHost(&s->h_state, sizeof(BuildState)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "pinned");
     if (rc == RTG_OK) {
         s->d_params = &s->d_state->params;
         s->d_work = &s->d_state->work;
     }
-    if (rc == RTG_OK && cudaMalloc(&s->d_ctr, sizeof(TraceCounters)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "ctr");
-    if (rc == RTG_OK && cudaMalloc(&s->d_ray_ctr, 8 * kRayCounters * sizeof(unsigned long long)) != cudaSuccess)
+    if (rc == RTG_OK && device_malloc(&s->d_ctr, sizeof(TraceCounters)) != cudaSuccess) rc = fail(RTG_NO_MEMORY, "ctr");
+    if (rc == RTG_OK && device_malloc(&s->d_ray_ctr, 8 * kRayCounters * sizeof(unsigned long long)) != cudaSuccess)
         rc = fail(RTG_NO_MEMORY, "ray counters");
     if (rc == RTG_OK && s->tune.heavy_cell > 0 &&
-        cudaMalloc(&s->d_defer, kDeferAlloc) != cudaSuccess) {
+        device_malloc(&s->d_defer, kDeferAlloc) != cudaSuccess) {
         s->d_defer = nullptr;
         rc = fail(RTG_NO_MEMORY, "deferred-ray queues");
     }
@@ -375,7 +390,7 @@ rtg_status rtg_scene_destroy(rtg_scene s) {
     cudaFree(s->d_qm);
     cudaFree(s->d_ql);
     cudaFree(s->d_io);
-    if (s->render_pool) cudaMemPoolDestroy(s->render_pool);
+    drop_render_pool(s);
     cudaFree(s->d_ctr);
     cudaFree(s->d_verts_back);
     if (s->copy_stream) cudaStreamSynchronize(s->copy_stream);
@@ -560,7 +575,7 @@ static bool grow_spheres(rtg_scene s) {
     cudaFree(s->d_csph);   // the build just read did not fit it: the grid names no spheres
     s->d_csph = nullptr;
     s->csph_cap = 0;
-    if (cudaMalloc(&s->d_csph, (size_t)n * sizeof(float4)) != cudaSuccess) {
+    if (device_malloc(&s->d_csph, (size_t)n * sizeof(float4)) != cudaSuccess) {
         cudaGetLastError();   // without them the block-per-ray pass reads the records
         s->d_csph = nullptr;
         return false;
@@ -1090,12 +1105,12 @@ rtg_status rtg_batch_create(const rtg_scene* scenes, int32_t nscenes, const int3
     b->ntasks = (int)ht.size();
     b->total = first;
     rtg_status rc = RTG_OK;
-    if (cudaMalloc(&b->d_build, sizeof(BuildArgs) * nscenes) != cudaSuccess ||
-        cudaMalloc(&b->d_scenes, sizeof(BatchScene) * nscenes) != cudaSuccess ||
-        cudaMalloc(&b->d_tasks, sizeof(BatchTask) * (ht.size() + 1)) != cudaSuccess ||
-        cudaMalloc(&b->d_counter, 3 * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&b->d_defer, sizeof(int2) * kDeferCap) != cudaSuccess ||
-        cudaMalloc(&b->d_first, sizeof(int) * kBuildKinds * (nscenes + 1)) != cudaSuccess)
+    if (device_malloc(&b->d_build, sizeof(BuildArgs) * nscenes) != cudaSuccess ||
+        device_malloc(&b->d_scenes, sizeof(BatchScene) * nscenes) != cudaSuccess ||
+        device_malloc(&b->d_tasks, sizeof(BatchTask) * (ht.size() + 1)) != cudaSuccess ||
+        device_malloc(&b->d_counter, 3 * sizeof(unsigned long long)) != cudaSuccess ||
+        device_malloc(&b->d_defer, sizeof(int2) * kDeferCap) != cudaSuccess ||
+        device_malloc(&b->d_first, sizeof(int) * kBuildKinds * (nscenes + 1)) != cudaSuccess)
         rc = fail(RTG_NO_MEMORY, "batch tables");
     if (rc == RTG_OK && ht.size() &&
         cudaMemcpy(b->d_tasks, ht.data(), sizeof(BatchTask) * ht.size(), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1219,7 +1234,7 @@ rtg_status rtg_scene_set_tuning(rtg_scene s, int32_t key, int32_t value) {
             if (value < 0) return fail(RTG_INVALID_PARAM, "heavy-cell threshold must be >= 0");
             if (value > 0 && !s->d_defer) {
                 CUDA_TRY(cudaSetDevice(s->device));
-                if (cudaMalloc(&s->d_defer, kDeferAlloc) != cudaSuccess) {
+                if (device_malloc(&s->d_defer, kDeferAlloc) != cudaSuccess) {
                     s->d_defer = nullptr;
                     return fail(RTG_NO_MEMORY, "deferred-ray queues");
                 }

@@ -185,9 +185,9 @@ rtg_status rtg_instances_create(const rtg_instance* inst, int32_t n, rtg_instanc
     set->device = dev;
     set->num_sms = inst[0].scene->num_sms;
     set->tune = inst[0].scene->tune;
-    if (cudaMalloc(&set->d_recs, sizeof(InstanceRec) * (size_t)n) != cudaSuccess ||
-        cudaMalloc(&set->d_params, instance_params_bytes(n)) != cudaSuccess ||
-        cudaMalloc(&set->d_counter, sizeof(unsigned long long) * kInstCounters) != cudaSuccess) {
+    if (device_malloc(&set->d_recs, sizeof(InstanceRec) * (size_t)n) != cudaSuccess ||
+        device_malloc(&set->d_params, instance_params_bytes(n)) != cudaSuccess ||
+        device_malloc(&set->d_counter, sizeof(unsigned long long) * kInstCounters) != cudaSuccess) {
         rtg_instances_destroy(set);
         return ifail(RTG_NO_MEMORY, "instances: device tables");
     }

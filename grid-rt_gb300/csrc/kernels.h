@@ -83,6 +83,13 @@ void launch_build_batch(const BuildArgs* d_tasks, int ntasks, const BatchGrid& g
 // the device flags ST_AMBIGUOUS); defined in api.cu.
 void host_resolve(GridParams& p, int32_t k, int64_t ntris, int64_t cell_cap);
 // Sets the text rtg_last_error() returns on this thread; defined in api.cu.
+// cudaMalloc; before it is refused, what the device's scenes keep of their render
+// buffers between frames is given back (shade.cu).
+cudaError_t device_malloc_bytes(void** p, size_t bytes);
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes) {
+    return device_malloc_bytes(reinterpret_cast<void**>(p), bytes);
+}
 void set_last_error(const std::string& msg);
 cudaError_t build_setup_attributes(int bitmap_words);
 

@@ -39,7 +39,7 @@ extern "C" rtg_status rtg_probe_read_gbs(int32_t device, int64_t bytes, int32_t 
     const int64_t n = bytes / 16;
     float4* buf = nullptr;
     float* out = nullptr;
-    if (cudaMalloc(&buf, (size_t)n * 16) != cudaSuccess || cudaMalloc(&out, sizeof(float)) != cudaSuccess) {
+    if (gridrt::device_malloc(&buf, (size_t)n * 16) != cudaSuccess || gridrt::device_malloc(&out, sizeof(float)) != cudaSuccess) {
         cudaFree(buf);
         gridrt::set_last_error("probe: allocation");
         return RTG_NO_MEMORY;

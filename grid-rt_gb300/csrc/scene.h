@@ -74,9 +74,10 @@ struct rtg_scene_s {
     gridrt::GridParams hp{};   // host copy of the last successful build
 
     // rtg_render's buffers: a pool of the scene's own, made by its first frame
-    // and destroyed with it, that keeps up to kRenderKeep bytes between frames
+    // and destroyed with it; the bytes it keeps (under shade.cu's lock)
     std::once_flag render_once;
     cudaMemPool_t render_pool = nullptr;
+    uint64_t render_kept = 0;
     unsigned char* d_io = nullptr;
     int64_t io_cap = 0;
     // rtg_trace_frame_async: shadow-ray area + two output slots, copied back
@@ -101,6 +102,8 @@ constexpr int32_t kHugeCap = 8192;      // rays a launch can hand to the block-p
 constexpr size_t kDeferAlloc = sizeof(int2) * (size_t)kRayCounters * (kDeferCap + kHugeCap);
 // Read-only device view of a built scene (for the trace kernels).
 SceneView scene_view(rtg_scene s);
+// Ends a scene's render buffers.
+void drop_render_pool(rtg_scene s);
 // Next per-launch counter slot (and deferred-ray queue) of the scene.
 TraceSlot scene_counter(rtg_scene s);
 // Camera checks and conversion shared by the camera-ray entry points.

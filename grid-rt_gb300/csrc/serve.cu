@@ -146,16 +146,16 @@ extern "C" rtg_status rtg_serve_run(const rtg_scene* scenes, int32_t nscenes, co
         cudaFree(d_pool);
         cudaFree(d_scenes);
     };
-    if (cudaMalloc(&d_pool, (size_t)pool.cap) != cudaSuccess || cudaMalloc(&d_scenes, sizeof(BatchScene) * nscenes))
+    if (device_malloc(&d_pool, (size_t)pool.cap) != cudaSuccess || device_malloc(&d_scenes, sizeof(BatchScene) * nscenes))
         rc = RTG_NO_MEMORY;
     for (Step& s : steps) {
         if (rc) break;
         if (cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming) != cudaSuccess ||
             cudaMallocHost(&s.h_tasks, sizeof(BatchTask) * kMaxStepTasks) != cudaSuccess ||
-            cudaMalloc(&s.d_tasks, sizeof(BatchTask) * kMaxStepTasks) != cudaSuccess ||
-            cudaMalloc(&s.d_counter, 3 * sizeof(unsigned long long)) != cudaSuccess ||
-            cudaMalloc(&s.d_defer, sizeof(int2) * kDeferCap) != cudaSuccess)
+            device_malloc(&s.d_tasks, sizeof(BatchTask) * kMaxStepTasks) != cudaSuccess ||
+            device_malloc(&s.d_counter, 3 * sizeof(unsigned long long)) != cudaSuccess ||
+            device_malloc(&s.d_defer, sizeof(int2) * kDeferCap) != cudaSuccess)
             rc = RTG_NO_MEMORY;
     }
     if (rc == RTG_OK) {

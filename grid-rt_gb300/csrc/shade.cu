@@ -15,6 +15,7 @@
 // + refracted x (1 - opacity).  vr::vec3f (vrbase) is not in the reference
 // checkout: a vector is normalised as v * (1 / sqrt(v.v)), dot products add
 // x, y, z left to right, one rounding per operation.
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -293,11 +294,17 @@ rtg_status sfail(rtg_status s, const std::string& msg) {
 // The scene's render buffers come from a pool of its own. The device's default
 // pool gives its memory back to the system at every wait, and a frame waits
 // once a level, so mapping it again was what a small frame spent most of its
-// time on: 640 x 480, three levels, 1,036 -> 671 us (a new scene's
-// first frame 1,543 -> 891). A host that
-// renders larger frames than kRenderKeep bytes hold maps the rest again each
-// time. Safe from several threads and streams: the pool orders reuse.
+// time on: 640 x 480, three levels, 1,036 -> 671 us (a new scene's first frame
+// 1,543 -> 891). The pools of a device keep up to kRenderKeep bytes between
+// frames: beyond that the scenes that rendered least recently give theirs back,
+// and larger frames map the rest again each time. (One pool for all scenes made
+// three scenes' frames in turn take 745 us instead of 652: memory that another
+// stream freed.) Safe from several threads and streams: a pool orders reuse,
+// and giving back takes only what is not in use.
 constexpr uint64_t kRenderKeep = 1ull << 30;
+
+std::mutex g_render_mutex;               // the list, and its scenes' render_kept
+std::vector<rtg_scene> g_rendered;       // scenes with a pool, least recently rendered first
 
 cudaMemPool_t render_pool(rtg_scene s) {
     std::call_once(s->render_once, [s] {
@@ -315,11 +322,61 @@ cudaMemPool_t render_pool(rtg_scene s) {
             cudaGetLastError();
         }
         cudaThreadExchangeStreamCaptureMode(&mode);
+        if (s->render_pool) {
+            std::lock_guard<std::mutex> lock(g_render_mutex);
+            g_rendered.push_back(s);
+        }
     });
     return s->render_pool;
 }
 
+// After a frame: what the scene's pool keeps, and the bound on the device's.
+void keep_render_buffers(rtg_scene s) {
+    if (!s->render_pool) return;
+    std::lock_guard<std::mutex> lock(g_render_mutex);
+    if (cudaMemPoolGetAttribute(s->render_pool, cudaMemPoolAttrReservedMemCurrent, &s->render_kept) != cudaSuccess)
+        cudaGetLastError();
+    g_rendered.erase(std::find(g_rendered.begin(), g_rendered.end(), s));
+    g_rendered.push_back(s);
+    uint64_t total = 0;
+    for (rtg_scene o : g_rendered) total += o->device == s->device ? o->render_kept : 0;
+    for (rtg_scene o : g_rendered) {
+        if (total <= kRenderKeep || o == s) break;
+        if (o->device != s->device || !o->render_kept) continue;
+        cudaMemPoolTrimTo(o->render_pool, 0);
+        total -= o->render_kept;
+        o->render_kept = 0;
+    }
+}
+
 }  // namespace
+
+namespace gridrt {
+void drop_render_pool(rtg_scene s) {
+    if (!s->render_pool) return;
+    std::lock_guard<std::mutex> lock(g_render_mutex);
+    g_rendered.erase(std::find(g_rendered.begin(), g_rendered.end(), s));
+    cudaMemPoolDestroy(s->render_pool);
+    s->render_pool = nullptr;
+}
+
+cudaError_t device_malloc_bytes(void** p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    int device = 0;
+    if (e != cudaErrorMemoryAllocation || cudaGetDevice(&device) != cudaSuccess) return e;
+    bool given = false;
+    std::lock_guard<std::mutex> lock(g_render_mutex);
+    for (rtg_scene s : g_rendered) {
+        if (s->device != device || !s->render_kept) continue;
+        cudaMemPoolTrimTo(s->render_pool, 0);
+        s->render_kept = 0;
+        given = true;
+    }
+    if (!given) return e;
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
+}
+}  // namespace gridrt
 
 extern "C" rtg_status rtg_render(rtg_scene s, const rtg_camera* cam, const rtg_shading* sh, float* d_rgb,
                                  int64_t* rays_out, void* stream) {
@@ -355,6 +412,7 @@ extern "C" rtg_status rtg_render(rtg_scene s, const rtg_camera* cam, const rtg_s
     auto cleanup = [&]() {
         for (void* p : owned) cudaFreeAsync(p, st);
         cudaStreamSynchronize(st);
+        keep_render_buffers(s);
     };
     rtg_material* d_mats = nullptr;
     rtg_point_light* d_lights = nullptr;

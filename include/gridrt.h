@@ -132,7 +132,11 @@ rtg_status rtg_scene_deform_vertices(rtg_scene scene, const float* d_base, const
 /* ---- grid build (UniformGridAccStructBuilder::buildGeometry) -------------
  * k = cells per triangle (the reference hard-codes 6,
  * src/rtplugins/UniformGridAccStructBuilder.cpp:91).  Synchronous: returns
- * after the grid is complete, growing device buffers as needed. */
+ * after the grid is complete, growing device buffers as needed.  The first
+ * build of a scene of at most 1,048,576 triangles with a list above 4,096
+ * entries also makes room for its lists' bounding spheres (16 bytes per
+ * reference the id buffers hold) and builds once more; without that memory,
+ * traces of it are slower. */
 rtg_status rtg_scene_build(rtg_scene scene, int32_t k, void* stream);
 /* Asynchronous build for graph capture and pipelining: enqueues the build
  * using the current buffer capacities (the first build of a scene runs
@@ -373,7 +377,9 @@ typedef struct {
 } rtg_shading;
 /* d_rgb: width x height x 3 float32, row-major from the bottom row (the
  * camera's pixel order, scanline).  rays_out (optional): rays traced in total
- * (primary, shadow, reflected, refracted). */
+ * (primary, shadow, reflected, refracted).  A device's scenes keep up to 1 GiB
+ * of their frames' buffers between frames; an allocation of this library that
+ * finds no memory takes it first. */
 rtg_status rtg_render(rtg_scene scene, const rtg_camera* cam, const rtg_shading* shading, float* d_rgb,
                       int64_t* rays_out, void* stream);
 
