@@ -250,6 +250,7 @@ TraceSlot scene_counter(rtg_scene s) {
     t.defer = s->d_defer ? s->d_defer + (size_t)slot * kDeferCap : nullptr;
     t.defer_cap = s->d_defer ? kDeferCap : 0;
     t.longest = s->hp.max_list < 0x7fffffffu ? (int32_t)s->hp.max_list : 0x7fffffff;
+    t.grid = &s->hp;
     // the block-per-ray pass is launched for scenes whose last checked build
     // had a list above kHugeList (the group pass handles such lists anyway)
     if (s->d_defer && s->hp.max_list > (uint32_t)kHugeList) {
@@ -798,6 +799,34 @@ bool camera_ok(const rtg_camera* cam) {
     if ((int64_t)cam->width * cam->height > ((int64_t)1 << 31)) return false;
     if (cam->order == RTG_ORDER_MORTON8 && ((cam->width & 7) || (cam->height & 7))) return false;
     return cam->order == RTG_ORDER_SCANLINE || cam->order == RTG_ORDER_MORTON8;
+}
+
+double image_share(const CameraArgs& cam, const float bmin[3], const float bmax[3]) {
+    // a corner at eye + x base + y nu + z nv is seen at (y / x, z / x)
+    const float *a = cam.base, *b = cam.nu, *c = cam.nv;
+    auto cross = [](const float* u, const float* v, int i) {
+        const int j = (i + 1) % 3, k = (i + 2) % 3;
+        return (double)u[j] * v[k] - (double)u[k] * v[j];
+    };
+    double lo[2] = {1.0, 1.0}, hi[2] = {0.0, 0.0};
+    for (int corner = 0; corner < 8; ++corner) {
+        double x = 0.0, y = 0.0, z = 0.0, det = 0.0;
+        for (int i = 0; i < 3; ++i) {
+            const double p = (double)((corner >> i) & 1 ? bmax[i] : bmin[i]) - cam.eye[i];
+            x += p * cross(b, c, i);
+            y += p * cross(c, a, i);
+            z += p * cross(a, b, i);
+            det += a[i] * cross(b, c, i);
+        }
+        if (!(x * det > 0.0)) return 0.0;
+        const double at[2] = {y / x, z / x};
+        for (int i = 0; i < 2; ++i) {
+            lo[i] = std::fmin(lo[i], std::fmax(at[i], 0.0));
+            hi[i] = std::fmax(hi[i], std::fmin(at[i], 1.0));
+        }
+    }
+    const double share = (hi[0] - lo[0]) * (hi[1] - lo[1]);
+    return hi[0] > lo[0] && hi[1] > lo[1] ? share : 0.0;
 }
 
 CameraArgs camera_args(const rtg_camera* cam) {

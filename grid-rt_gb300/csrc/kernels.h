@@ -191,7 +191,11 @@ struct TraceSlot {
     int2* huge = nullptr; // {ray, cell} entries of rays at a list above kHugeList (nullptr: no block pass)
     int32_t huge_cap = 0;
     int32_t longest = 0x7fffffff;   // longest list of the scene's last checked build (unknown: the largest value)
+    const GridParams* grid = nullptr;   // that build's parameters (read by the launching call only)
 };
+// Share of the image that the rectangle around a box's projection covers; 0 when
+// part of the box lies beside or behind the eye.
+double image_share(const CameraArgs& cam, const float bmin[3], const float bmax[3]);
 // Lists longer than this are tested by a whole block (the block-per-ray pass)
 // when the trace's slot has a huge-list queue.
 static constexpr int32_t kHugeList = 2048;

@@ -1682,6 +1682,28 @@ inline int32_t work_mult(long long n, int sms) {
     return (int32_t)(m < 4 ? 4 : (m > kHeavyWorkMult ? kHeavyWorkMult : m));
 }
 
+// Lanes per ray of a camera or frame launch that lanes_for gives 8.  Beyond the
+// resident lanes that pays while enough of the rays miss the scene's box or walk
+// far in it.  A small mesh that fills the image does better by one ray a lane as
+// soon as more rays than the resident lanes can meet its box, the smallest ones
+// (walks of a few cells) at four fifths; their camera launches, which end with
+// the hit, by 6/4 and 5/4 of the lanes at the latest.  us at 8 lanes and at one,
+// frames: 229 x 915, the sphere filling the image, 2,352 triangles 97 and 87,
+// 9,312 130 and 109; 256 x 1,024, 25,760 triangles 197 and 134; 260 x 1,040,
+// plane and debris of 2,000 triangles 111 and 98, of 20,000 (127,000 rays at the
+// box) 178 and 238; 200 x 800 (105,000 at the sphere's) 81 and 86.  Camera
+// launches, plane and debris of 2,000 triangles: 224 x 896 69 and 65, 256 x 1,024
+// 87 and 69; of 5,000: 224 x 896 76 and 79, 256 x 1,024 95 and 81.
+static constexpr int64_t kFewTris = 32768, kFewestTris = 4096;
+inline int image_lanes(const TraceIO& io, const TraceSlot& slot, bool frame, int num_sms) {
+    if (!slot.grid || slot.grid->ntris > kFewTris) return 8;
+    const bool fewest = slot.grid->ntris <= kFewestTris;
+    const long long resident = 1024LL * num_sms;
+    if (!frame && 4 * io.n > (fewest ? 5 : 6) * resident) return 1;
+    const double meet = (double)io.n * image_share(io.cam, slot.grid->bmin, slot.grid->bmax);
+    return meet > (fewest ? 0.8 : 1.0) * (double)resident ? 1 : 8;
+}
+
 template <int MODE>
 inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, const TraceTuning& tune, int num_sms,
                         cudaStream_t st) {
@@ -1700,7 +1722,8 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
         const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms));
         io.work = less > few ? less : few;
     }
-    const int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera ? 7 : MODE == MODE_ANY ? 3 : 4));
+    int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera ? 7 : MODE == MODE_ANY ? 3 : 4));
+    if (camera && lanes == 8 && io.n > 1024LL * num_sms / 2) lanes = image_lanes(io, slot, MODE == MODE_FRAME, num_sms);
     if (lanes > 1) {
         // every ray walked by a group of lanes from its start.  Groups of 16
         // and 32 deal any list out themselves, as do groups of 8 when no list
