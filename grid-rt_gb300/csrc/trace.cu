@@ -141,11 +141,12 @@ __global__ void __launch_bounds__(128, GRIDRT_TRACE_MIN_BLOCKS)
         io.work = work_limit(io.heavy, kHeavyWorkMult);
         io.defer_base = (int32_t)T.first;
         io.refill = refill;
+        io.alike = 7;
         io.any = T.mode == MODE_ANY;
         io.occ = static_cast<uint8_t*>(T.out);
         io.hits = static_cast<int4*>(T.out);
         const int32_t base = (int32_t)((long long)b - T.first);
-        if (refill > 0 && !chunk_coherent(P[T.scene], io, base)) {
+        if (refill > 0 && !chunk_coherent<true>(P[T.scene], io, base)) {
             b = trace_task_refill<ER>(P[T.scene], V, io, L, T.first, base, cells, tests, started);
         } else {
             trace_batch32<MODE_TASK, ER>(P[T.scene], V, io, L, base, cells, tests, started);

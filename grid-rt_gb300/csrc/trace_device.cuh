@@ -549,6 +549,7 @@ struct TraceIO {
     int32_t work;                  // and rays with more tests than this
     int32_t defer_base;            // added to a deferred ray's index (a batch task's first)
     int32_t refill;                // > 0: lane refill at this many idle lanes (trace_refill)
+    int32_t alike;                 // eighths of a chunk's rays that must be like the ray before them (chunk_alike)
     int any;                       // TASK: occlusion (else closest hits)
     int2* huge;                    // rays at a list above kHugeList, for the block pass (nullptr: none)
     int32_t huge_cap;
@@ -771,16 +772,20 @@ constexpr int trace_min_blocks(int mode, int tpb) {
 }
 
 // Whether the 32 rays from `base` walk alike: of those that follow another ray,
-// 7 in 8 start within a few cells of it and go within a narrow cone of the first
-// ray's direction (camera rays, shadow rays of one surface or two).  Slots
-// without a shadow ray (tfar < 0) are neither.  1024^2 shadow rays of the sphere
-// and of plane and debris, scanline, 135 and 227 us; every origin against the
-// first slot's, which may hold no ray, 178 and 222; half of the pairs 135 and
-// 258.  Two cells: the sphere's 640 x 480 in Morton order 95 -> 119; a cone of
-// 0.05: its camera rays 192 -> 235; of 0.15, or of each ray's predecessor: 64
-// scenes in one batch, images of 50 to 400 pixels a row, 2,514 -> 2,539 and 2,565.
-// One component at a time: the lanes' walks are live around it.
-static __device__ __noinline__ bool chunk_alike(float cx, float cy, float cz, const float4* rays, int32_t n, int32_t base) {
+// most start within a few cells of it and go within a narrow cone of its
+// direction (camera rays, shadow rays of one surface or two); in a batch's task,
+// of the first ray's direction.  Slots without a shadow ray (tfar < 0) are
+// neither.  1024^2 shadow rays of the sphere and of plane and debris, scanline,
+// 135 and 228 us; every origin against the first slot's, which may hold no ray,
+// 178 and 222; pairs within two cells and 0.05 134 and 255 at half of them.
+// Directions against the first ray's: camera rays of 540 x 540 pixels, whose rows
+// end within a chunk, 100 us for 74 (25,760 triangles: 167 for 141); but 64
+// scenes in one batch, images of 50 to 400 pixels a row, 2,514 for 2,565, which
+// are the better by refill.  One component at a time: the lanes' walks are live
+// around it.
+template <bool TASK>
+static __device__ __noinline__ bool chunk_alike(float cx, float cy, float cz, const float4* rays, int32_t n, int32_t base,
+                                                int32_t eighths) {
     const int32_t r = min(base + (int32_t)(threadIdx.x & 31), n - 1);
     const float* __restrict__ q = reinterpret_cast<const float*>(rays + 2 * (int64_t)r);
     const float cell[3] = {cx, cy, cz};
@@ -791,15 +796,17 @@ static __device__ __noinline__ bool chunk_alike(float cx, float cy, float cz, co
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const float o = __ldg(q + a), d = __ldg(q + 4 + a);
-        const float o0 = __shfl_up_sync(FULL, o, 1), d0 = __shfl_sync(FULL, d, first);
+        const float o0 = __shfl_up_sync(FULL, o, 1);
+        const float d0 = TASK ? __shfl_sync(FULL, d, first) : __shfl_up_sync(FULL, d, 1);
         if (!(fabsf(o - o0) <= kChunkCells * cell[a])) alike = false;
         off += fabsf(d - d0);
         len += fabsf(d0);
     }
-    return 8 * __popc(__ballot_sync(FULL, alike && off <= kChunkCone * len) & pairs) >= 7 * __popc(pairs);
+    return 8 * __popc(__ballot_sync(FULL, alike && off <= kChunkCone * len) & pairs) >= eighths * __popc(pairs);
 }
+template <bool TASK>
 __device__ __forceinline__ bool chunk_coherent(const SParams& P, const TraceIO& io, int32_t base) {
-    return chunk_alike(P.cell[0], P.cell[1], P.cell[2], io.rays, (int32_t)io.n, base);
+    return chunk_alike<TASK>(P.cell[0], P.cell[1], P.cell[2], io.rays, (int32_t)io.n, base, io.alike);
 }
 
 // Lane refill for incoherent rays: instead of tracing a claimed batch of 32 to
@@ -886,7 +893,7 @@ __global__ void __launch_bounds__(TPB, trace_min_blocks(MODE, TPB)) trace_kernel
     // the launch's rays lane by lane
     constexpr bool kArrays = MODE == MODE_NEAREST || MODE == MODE_ANY;
     while ((long long)b < io.n) {
-        if (io.refill > 0 && !(kArrays && chunk_coherent(P, io, (int32_t)b))) {
+        if (io.refill > 0 && !(kArrays && chunk_coherent<false>(P, io, (int32_t)b))) {
             trace_refill<MODE, ER>(P, s, io, L, b, cells, tests, started);
             break;
         }
@@ -1671,6 +1678,13 @@ inline void launch_huge(const SceneView& s, const TraceIO& io, int num_sms, cuda
     launch_k(trace_huge_kernel<MODE, COUNT>, (unsigned)(per_sm * num_sms), kHugeThreads, kStageBytes, st, s, io);
 }
 
+// The eighths of a chunk's rays that must be like the ray before them for the
+// chunk to walk by whole lists: half in launches of a few chunks a warp, which
+// end with their longest rays, 7 beyond.  Shadow rays of 512^2 images given as
+// an array, us at 7 and at 4: plane and debris of 2,000 triangles 52 and 46, of
+// 5,000 70 and 58; of 1024^2 images: 100,000 triangles 227 and 258.
+inline int32_t alike_eighths(long long n, int sms) { return n <= 2048LL * sms ? 4 : 7; }
+
 // The tests after which a camera ray (with its shadow ray in a frame) is handed
 // to a group of lanes, in heavy-cell thresholds: the fewer the shorter the tail
 // of a launch, but its queue is fixed, so larger launches hand on fewer of
@@ -1717,6 +1731,7 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
     io.huge = defer ? slot.huge : nullptr;
     io.huge_cap = io.huge ? slot.huge_cap : 0;
     cudaMemsetAsync(slot.ctr, 0, 8 * sizeof(unsigned long long), st);
+    io.alike = alike_eighths(io.n, num_sms);
     io.work = work_limit(io.heavy, kHeavyWorkMult);
     if (camera && io.heavy != kNoHeavy) {   // below 128 tests only where the caller's threshold says so
         const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms));
