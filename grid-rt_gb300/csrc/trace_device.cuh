@@ -45,7 +45,7 @@ static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the group-of-lanes pass
 static constexpr int32_t kNoHeavy = 0x7fffffff;
 // A ray is also deferred once its tests would pass kHeavyWorkMult x the
-// heavy-cell threshold in total (frames: work_mult).
+// heavy-cell threshold in total (smaller launches: work_mult).
 static constexpr int32_t kHeavyWorkMult = 8;
 
 
@@ -1685,14 +1685,16 @@ inline void launch_huge(const SceneView& s, const TraceIO& io, int num_sms, cuda
 // 5,000 70 and 58; of 1024^2 images: 100,000 triangles 227 and 258.
 inline int32_t alike_eighths(long long n, int sms) { return n <= 2048LL * sms ? 4 : 7; }
 
-// The tests after which a camera ray (with its shadow ray in a frame) is handed
-// to a group of lanes, in heavy-cell thresholds: the fewer the shorter the tail
-// of a launch, but its queue is fixed, so larger launches hand on fewer of
-// their rays.  Frames of the sphere / of plane and debris, us at 8 -> here:
-// 518,400 pixels 166 -> 133 / 398 -> 367 (4), 1,048,576 207 -> 186 /
-// 526 -> 530 (5).  Ray arrays stay at 8 (4 M random rays 2,254 us, at 4 2,321).
-inline int32_t work_mult(long long n, int sms) {
-    const long long m = 2 + n / (2048LL * sms);
+// The tests after which a ray (a frame's with its shadow ray) is handed to a group
+// of lanes, in heavy-cell thresholds: the fewer the shorter the tail of a launch,
+// but its queue is fixed, so larger launches hand on fewer of their rays.
+// Frames of the sphere / of plane and debris, us at 8 -> here: 518,400 pixels
+// 166 -> 133 / 398 -> 367 (4), 1,048,576 207 -> 186 / 526 -> 530 (5).  Arrays come
+// to 8 at four times the resident lanes (4 M random rays 2,254 us, at 4 2,321);
+// 262,144 random rays in plane and debris of 2,000 / 65,536 triangles 132 -> 114 /
+// 299 -> 284, segments 166 -> 146 / 369 -> 352 (4).
+inline int32_t work_mult(long long n, int sms, bool camera) {
+    const long long m = camera ? 2 + n / (2048LL * sms) : 2 * n / (1024LL * sms);
     return (int32_t)(m < 4 ? 4 : (m > kHeavyWorkMult ? kHeavyWorkMult : m));
 }
 
@@ -1733,8 +1735,8 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
     cudaMemsetAsync(slot.ctr, 0, 8 * sizeof(unsigned long long), st);
     io.alike = alike_eighths(io.n, num_sms);
     io.work = work_limit(io.heavy, kHeavyWorkMult);
-    if (camera && io.heavy != kNoHeavy) {   // below 128 tests only where the caller's threshold says so
-        const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms));
+    if (io.heavy != kNoHeavy) {   // below 128 tests only where the caller's threshold says so
+        const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms, camera));
         io.work = less > few ? less : few;
     }
     int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera ? 7 : MODE == MODE_ANY ? 3 : 4));
