@@ -1685,6 +1685,16 @@ inline void launch_huge(const SceneView& s, const TraceIO& io, int num_sms, cuda
 // 5,000 70 and 58; of 1024^2 images: 100,000 triangles 227 and 258.
 inline int32_t alike_eighths(long long n, int sms) { return n <= 2048LL * sms ? 4 : 7; }
 
+// Whether rays through the scene make some 256 tests and more (references a cell,
+// over half the cells along the axes: a soup of triangles as large as its box's
+// cells makes 1,500, plane and debris of 100,000 triangles 110 to 160).  Not those
+// whose references lie in a few crowded cells (a step of the skewed scene would
+// take 1,676 us for 1,646).
+inline bool dense_scene(const GridParams* g) {
+    return g && g->ncells > 0 && g->max_list <= (uint32_t)kHugeList &&
+           0.5 * (double)g->nrefs * ((double)g->res[0] + g->res[1] + g->res[2]) > 256.0 * (double)g->ncells;
+}
+
 // The tests after which a ray (a frame's with its shadow ray) is handed to a group
 // of lanes, in heavy-cell thresholds: the fewer the shorter the tail of a launch,
 // but its queue is fixed, so larger launches hand on fewer of their rays.
@@ -1693,7 +1703,11 @@ inline int32_t alike_eighths(long long n, int sms) { return n <= 2048LL * sms ? 
 // to 8 at four times the resident lanes (4 M random rays 2,254 us, at 4 2,321);
 // 262,144 random rays in plane and debris of 2,000 / 65,536 triangles 132 -> 114 /
 // 299 -> 284, segments 166 -> 146 / 369 -> 352 (4).
-inline int32_t work_mult(long long n, int sms, bool camera) {
+// Camera and frame launches stay at 8 in dense scenes, where every ray is one of
+// those: 640 x 640 camera rays / frames of a soup of 20,000 triangles 206 -> 186 /
+// 392 -> 329, of 5,000 800 x 800 192 / 400 -> 291.
+inline int32_t work_mult(long long n, int sms, bool camera, const GridParams* grid) {
+    if (camera && dense_scene(grid)) return kHeavyWorkMult;
     const long long m = camera ? 2 + n / (2048LL * sms) : 2 * n / (1024LL * sms);
     return (int32_t)(m < 4 ? 4 : (m > kHeavyWorkMult ? kHeavyWorkMult : m));
 }
@@ -1709,12 +1723,16 @@ inline int32_t work_mult(long long n, int sms, bool camera) {
 // plane and debris of 2,000 triangles 111 and 98, of 20,000 (127,000 rays at the
 // box) 178 and 238; 200 x 800 (105,000 at the sphere's) 81 and 86.  Camera
 // launches, plane and debris of 2,000 triangles: 224 x 896 69 and 65, 256 x 1,024
-// 87 and 69; of 5,000: 224 x 896 76 and 79, 256 x 1,024 95 and 81.
+// 87 and 69; of 5,000: 224 x 896 76 and 79, 256 x 1,024 95 and 81.  In dense
+// scenes a lane a ray keeps the GPU busy beyond the resident lanes: 512 x 512
+// frames of soups of 20,000 / 60,000 triangles 273 and 238 / 431 and 393, of
+// 440 x 440 pixels 215 and 206 / 333 and 318.
 static constexpr int64_t kFewTris = 32768, kFewestTris = 4096;
 inline int image_lanes(const TraceIO& io, const TraceSlot& slot, bool frame, int num_sms) {
+    const long long resident = 1024LL * num_sms;
+    if (io.n > resident && dense_scene(slot.grid)) return 1;
     if (!slot.grid || slot.grid->ntris > kFewTris) return 8;
     const bool fewest = slot.grid->ntris <= kFewestTris;
-    const long long resident = 1024LL * num_sms;
     if (!frame && 4 * io.n > (fewest ? 5 : 6) * resident) return 1;
     const double meet = (double)io.n * image_share(io.cam, slot.grid->bmin, slot.grid->bmax);
     return meet > (fewest ? 0.8 : 1.0) * (double)resident ? 1 : 8;
@@ -1736,7 +1754,7 @@ inline void launch_mode(const SceneView& s, TraceIO io, const TraceSlot& slot, c
     io.alike = alike_eighths(io.n, num_sms);
     io.work = work_limit(io.heavy, kHeavyWorkMult);
     if (io.heavy != kNoHeavy) {   // below 128 tests only where the caller's threshold says so
-        const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms, camera));
+        const int32_t few = io.work < 128 ? io.work : 128, less = work_limit(io.heavy, work_mult(io.n, num_sms, camera, slot.grid));
         io.work = less > few ? less : few;
     }
     int lanes = io.ctr ? 1 : (tune.lanes ? tune.lanes : lanes_for(io.n, num_sms, camera ? 7 : MODE == MODE_ANY ? 3 : 4));
