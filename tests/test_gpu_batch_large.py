@@ -53,3 +53,37 @@ def test_occlusion_with_a_tmax_that_is_not_a_number(gridlib, refill):
     b.trace_async()
     assert b.check() == 0
     assert np.array_equal(outs[0].cpu().numpy()[:, 0], want)
+
+
+@pytest.mark.parametrize("cell_records,heavy,refill",
+                         [(False, 0, 0), (True, 32, 0), (False, 4, 0), (True, 32, 8), (False, 4, 16), (False, 0, 1)])
+def test_large_batch_equals_scene_traces(gridlib, cell_records, heavy, refill):
+    """With and without cell-ordered records, hand-on and lane refill, against the
+    scenes' one-lane walks without them.  Every ray in the soup meets lists above 4,
+    so heavy = 4 also overfills the batch's queue of 65,536 rays."""
+    kinds = [scenes.tiny_scene(3, 20_000), scenes.plane_and_debris(seed=5, quads=30, debris=9000),
+             scenes.deforming_sphere(0), scenes.plane_and_debris(seed=6, quads=12, debris=300)]
+    sizes = [75_001, 40_003, *_sizes(2)]
+    scs, tasks, want = [], [], []
+    for i, (sc, n) in enumerate(zip(kinds, sizes)):
+        s = gridlib.Scene(0)
+        s.set_geometry(sc.verts, sc.idx)
+        s.set_tuning(lanes=1, heavy_cell=0, refill=0)
+        s.build(4)
+        rays, seg = _rays(sc, n, i), _rays(sc, n // 3 + 1, 50 + i, 0.5)
+        cam = scenes.camera_rays(scenes.plane_and_debris_camera(64, 64))[:len(rays) // 4]
+        rays[:len(cam)] = cam                                   # alike, then not
+        want += [s.trace_nearest(rays).view(np.int32), s.trace_any(seg)]
+        tasks += [(i, gridlib.RTG_MODE_NEAREST, rays), (i, gridlib.RTG_MODE_ANY, seg)]
+        if cell_records and i % 2 == 0:
+            s.set_tuning(cell_records=True)
+        scs.append(s)
+    b, _, outs = _batch(gridlib, scs, tasks)
+    b.set_tuning(heavy_cell=heavy, heavy_lanes=4 if heavy == 4 else 8, refill=refill)
+    for _ in range(2):
+        b.build_async()
+        b.trace_async()
+        assert b.check() == 0
+        for got, exp in zip(outs, want):
+            assert np.array_equal(got.cpu().numpy().reshape(exp.shape), exp)
+            got.fill_(77)

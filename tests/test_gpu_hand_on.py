@@ -55,3 +55,42 @@ def test_random_rays_beyond_the_resident_lanes(gridlib, mode):
     if mode == "nearest":
         assert as_set < 1.08 * early, (as_set, early)
     s.close()
+
+
+@pytest.mark.parametrize("heavy", [1, 4, 16, 64])
+def test_hand_on_of_the_one_lane_walk(gridlib, heavy):
+    """Rays handed on by one lane give the bits of the walk that hands none on, for
+    frames, camera rays and arrays; small thresholds also overfill the queue."""
+    import torch
+    sc = scenes.deforming_sphere(2)
+    cam = scenes.deforming_sphere_camera(512, 512)
+    n = 512 * 512
+    rays = scenes.random_rays(np.random.default_rng(11), 120_000, (-1.2, -1.2, -1.2), (1.2, 1.2, 1.2))
+    seg = rays.copy()
+    seg[:, 7] = 0.5
+    s = gridlib.Scene(0)
+    s.set_geometry(sc.verts, sc.idx)
+    s.set_tuning(lanes=1)
+
+    def results(order):
+        hits = torch.zeros((n, 4), dtype=torch.int32, device="cuda")
+        occ = torch.full((n,), 7, dtype=torch.uint8, device="cuda")
+        sr = torch.zeros((n, 8), dtype=torch.float32, device="cuda")
+        s.trace_frame_device(cam, scenes.SPHERE_LIGHT, hits, occ, sr, order=order)
+        hits2, sr2 = torch.zeros_like(hits), torch.zeros_like(sr)
+        s.trace_camera_device(cam, hits2, scenes.SPHERE_LIGHT, sr2, order=order)
+        torch.cuda.synchronize()
+        out = [x.cpu().numpy() for x in (hits, occ, sr, hits2, sr2)]
+        return [x.view(np.uint32) if x.dtype == np.float32 else x for x in out] + [
+            s.trace_nearest(rays).view(np.int32), s.trace_any(seg)]
+
+    s.set_tuning(heavy_cell=0, refill=0)
+    s.build(8)
+    want = {order: results(order) for order in ("scanline", "morton8")}
+    for records, lanes, refill in ((False, 8, 0), (True, 4, 16), (True, 16, 1), (False, 32, 8)):
+        s.set_tuning(heavy_cell=heavy, cell_records=records, heavy_lanes=lanes, refill=refill)
+        s.build(8)
+        for order in want:
+            for a, b in zip(want[order], results(order)):
+                assert np.array_equal(a, b), (records, lanes, refill, order)
+    s.close()
