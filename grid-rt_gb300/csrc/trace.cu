@@ -75,28 +75,7 @@ __device__ __forceinline__ unsigned long long trace_task_refill(const SParams& P
             continue;
         }
         bool fin = advance_two<MODE_TASK, ER>(P, L, s, active, cells, tests);
-        if (io.defer) {
-            const bool d = fin && L.id == kDeferred;
-            const unsigned m = __ballot_sync(FULL, d);
-            if (m) {
-                const int leader = __ffs(m) - 1;
-                unsigned long long slot0 = 0;
-                if (lane == leader) slot0 = atomicAdd(io.counter + 1, (unsigned long long)__popc(m));
-                slot0 = __shfl_sync(FULL, slot0, leader);
-                if (d) {
-                    const unsigned long long slot = slot0 + __popc(m & ((1u << lane) - 1u));
-                    if (slot < (unsigned long long)io.defer_cap) {
-                        io.defer[slot] = make_int2(defer_tag<MODE_TASK>(L, io),
-                                                   L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
-                        active = false;
-                    } else {
-                        set_deferral(L, kNoHeavy, kNoHeavy);
-                        L.id = -1;
-                    }
-                    fin = false;
-                }
-            }
-        }
+        if (io.defer) hand_on<MODE_TASK>(P, io, L, active, fin);
         if (fin) {
             finish_ray<MODE_TASK>(io, P, s, L);
             active = false;

@@ -701,6 +701,32 @@ __device__ __forceinline__ int32_t defer_tag(const Lane& L, const TraceIO& io) {
     return (MODE == MODE_FRAME && L.tmax > -kFltMax) ? -1 - L.ray : L.ray + io.defer_base;
 }
 
+// Hands on the lanes that stopped at a long list, or after many tests: one
+// atomicAdd for the warp's.  The walk resumes at the lane's cell in the
+// group-of-lanes pass.
+template <int MODE>
+__device__ __forceinline__ void hand_on(const SParams& P, const TraceIO& io, Lane& L, bool& active, bool& fin) {
+    const int lane = threadIdx.x & 31;
+    const bool d = fin && L.id == kDeferred;
+    const unsigned m = __ballot_sync(FULL, d);
+    if (!m) return;
+    const int leader = __ffs(m) - 1;
+    unsigned long long at = 0;
+    if (lane == leader) at = atomicAdd(io.counter + 1, (unsigned long long)__popc(m));
+    at = __shfl_sync(FULL, at, leader);
+    if (d) {
+        const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
+        if (slot < (unsigned long long)io.defer_cap) {
+            io.defer[slot] = make_int2(defer_tag<MODE>(L, io), L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
+            active = false;
+        } else {
+            set_deferral(L, kNoHeavy, kNoHeavy);   // queue full: the lane tests the cell itself
+            L.id = -1;
+        }
+        fin = false;
+    }
+}
+
 template <int MODE, int ER>
 __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView& s, const TraceIO& io, Lane& L,
                                               long long base, uint32_t& cells, uint32_t& tests, uint32_t& started) {
@@ -718,29 +744,7 @@ __device__ __forceinline__ void trace_batch32(const SParams& P, const SceneView&
     }
     while (__any_sync(FULL, active)) {
         bool fin = advance<MODE, ER>(P, L, s, active, cells, tests);
-        if (io.defer) {
-            // warp-aggregated push of the lanes that met a long list
-            const bool d = fin && L.id == kDeferred;
-            const unsigned m = __ballot_sync(FULL, d);
-            if (m) {
-                const int leader = __ffs(m) - 1;
-                unsigned long long at = 0;
-                if (lane == leader) at = atomicAdd(io.counter + 1, (unsigned long long)__popc(m));
-                at = __shfl_sync(FULL, at, leader);
-                if (d) {
-                    const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
-                    if (slot < (unsigned long long)io.defer_cap) {
-                        // the walk resumes at this cell in the group-of-lanes pass
-                        io.defer[slot] = make_int2(defer_tag<MODE>(L, io), L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
-                        active = false;
-                    } else {
-                        set_deferral(L, kNoHeavy, kNoHeavy);   // queue full: the lane tests the cell itself
-                        L.id = -1;
-                    }
-                    fin = false;
-                }
-            }
-        }
+        if (io.defer) hand_on<MODE>(P, io, L, active, fin);
         if (fin) active = finish_ray<MODE>(io, P, s, L);
     }
 }
@@ -851,28 +855,7 @@ __device__ __forceinline__ void trace_refill(const SParams& P, const SceneView& 
             continue;
         }
         bool fin = advance_two<MODE, ER>(P, L, s, active, cells, tests);
-        if (io.defer) {
-            const bool d = fin && L.id == kDeferred;
-            const unsigned m = __ballot_sync(FULL, d);
-            if (m) {
-                const int leader = __ffs(m) - 1;
-                unsigned long long at = 0;
-                if (lane == leader) at = atomicAdd(io.counter + 1, (unsigned long long)__popc(m));
-                at = __shfl_sync(FULL, at, leader);
-                if (d) {
-                    const unsigned long long slot = at + __popc(m & ((1u << lane) - 1u));
-                    if (slot < (unsigned long long)io.defer_cap) {
-                        io.defer[slot] = make_int2(defer_tag<MODE>(L, io),
-                                                   L.x + L.y * P.res[0] + L.z * P.res[0] * P.res[1]);
-                        active = false;
-                    } else {
-                        set_deferral(L, kNoHeavy, kNoHeavy);
-                        L.id = -1;
-                    }
-                    fin = false;
-                }
-            }
-        }
+        if (io.defer) hand_on<MODE>(P, io, L, active, fin);
         if (fin) active = finish_ray<MODE>(io, P, s, L);
     }
 }
