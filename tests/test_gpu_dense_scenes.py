@@ -1,25 +1,12 @@
 """Frames of a soup whose every ray meets hundreds of triangles: rays are not handed
 on as if they were the few long ones, and beyond the resident lanes one lane
 traces a ray; the results are those of tracing every ray to its end."""
-import time
-
 import pytest
 
+import timing
 from gridrt import scenes
 
 pytestmark = pytest.mark.gpu
-
-
-def _best(call, runs=60):
-    """Seconds of the shortest of `runs` calls, each waited for."""
-    import torch
-    best = float("inf")
-    for _ in range(runs):
-        t = time.perf_counter()
-        call()
-        torch.cuda.synchronize()
-        best = min(best, time.perf_counter() - t)
-    return best
 
 
 @pytest.mark.parametrize("part", [1.68, 4.1])
@@ -29,9 +16,11 @@ def test_frames_of_a_soup(gridlib, part):
     handing on after 512 tests at 4.1, 293 us against 400)."""
     import torch
     sc = scenes.tiny_scene(3, 5000)
-    s = gridlib.Scene(0)
-    s.set_geometry(sc.verts, sc.idx)
-    s.build(4)
+    s, told = gridlib.Scene(0), gridlib.Scene(0)
+    for x in (s, told):
+        x.set_geometry(sc.verts, sc.idx)
+        x.build(4)
+    told.set_tuning(lanes=1, heavy_cell=64)
     n = 1024 * torch.cuda.get_device_properties(0).multi_processor_count * part
     cam = scenes.look_at_camera((0.9, 0.6, 1.5), (0.0, 0.0, 0.0), (0.0, 1.0, 0.0), 60.0, int(n ** 0.5), int(n ** 0.5))
     m = cam.width * cam.height
@@ -39,17 +28,14 @@ def test_frames_of_a_soup(gridlib, part):
              torch.full((m,), x, dtype=torch.uint8, device="cuda"),
              torch.zeros((m, 8), dtype=torch.float32, device="cuda")) for x in (7, 8, 9)]
 
-    def frame(o):
-        s.trace_frame_device(cam, scenes.PLANE_LIGHT, *o)
+    def frame(x, o):
+        x.trace_frame_device(cam, scenes.PLANE_LIGHT, *o)
 
-    as_set = _best(lambda: frame(outs[0]))
-    s.set_tuning(lanes=1, heavy_cell=64)
-    other = _best(lambda: frame(outs[1]))
-    s.set_tuning(heavy_cell=0)
-    frame(outs[2])
+    slower = timing.ratio(lambda: frame(s, outs[0]), lambda: frame(told, outs[1]), 1.1)
+    told.set_tuning(heavy_cell=0)
+    frame(told, outs[2])
     torch.cuda.synchronize()
     for o in outs[:2]:
         for a, b in zip(o, outs[2]):
             assert torch.equal(a, b)
-    assert as_set < 1.1 * other, (as_set, other)
-    s.close()
+    assert slower < 1.1

@@ -1,26 +1,13 @@
 """Random rays of a launch a little larger than the GPU's resident lanes: those that
 meet many triangles are handed on early, so that the launch does not wait for
 them; the results are those of tracing every ray to its end."""
-import time
-
 import numpy as np
 import pytest
 
+import timing
 from gridrt import scenes
 
 pytestmark = pytest.mark.gpu
-
-
-def _best(call, runs=60):
-    """Seconds of the shortest of `runs` calls, each waited for."""
-    import torch
-    best = float("inf")
-    for _ in range(runs):
-        t = time.perf_counter()
-        call()
-        torch.cuda.synchronize()
-        best = min(best, time.perf_counter() - t)
-    return best
 
 
 @pytest.mark.parametrize("mode", ["nearest", "any"])
@@ -35,26 +22,25 @@ def test_random_rays_beyond_the_resident_lanes(gridlib, mode):
     if mode == "any":
         rays[:, 7] = 0.7
     rays = torch.from_numpy(rays).cuda()
-    s = gridlib.Scene(0)
-    s.set_geometry(sc.verts, sc.idx)
-    s.build(8)
+    s, early = gridlib.Scene(0), gridlib.Scene(0)
+    for x in (s, early):
+        x.set_geometry(sc.verts, sc.idx)
+        x.build(8)
+        x.set_tuning(lanes=1)
+    early.set_tuning(heavy_cell=16)          # 8 thresholds: 128 tests
     outs = [torch.full((n, 4) if mode == "nearest" else (n,), x,
                        dtype=torch.int32 if mode == "nearest" else torch.uint8, device="cuda") for x in (7, 8, 9)]
 
-    def trace(out):
-        return s.trace_nearest_device(rays, n, out) if mode == "nearest" else s.trace_any_device(rays, n, out)
+    def trace(x, out):
+        return x.trace_nearest_device(rays, n, out) if mode == "nearest" else x.trace_any_device(rays, n, out)
 
-    s.set_tuning(lanes=1)
-    as_set = _best(lambda: trace(outs[0]))
-    s.set_tuning(heavy_cell=16)              # 8 thresholds: 128 tests
-    early = _best(lambda: trace(outs[1]))
-    s.set_tuning(heavy_cell=0)
-    trace(outs[2])
+    slower = timing.ratio(lambda: trace(s, outs[0]), lambda: trace(early, outs[1]), 1.08)
+    early.set_tuning(heavy_cell=0)
+    trace(early, outs[2])
     torch.cuda.synchronize()
     assert torch.equal(outs[0], outs[2]) and torch.equal(outs[1], outs[2])
     if mode == "nearest":
-        assert as_set < 1.08 * early, (as_set, early)
-    s.close()
+        assert slower < 1.08
 
 
 @pytest.mark.parametrize("heavy", [1, 4, 16, 64])

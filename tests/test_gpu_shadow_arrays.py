@@ -1,25 +1,24 @@
 """The shadow rays a camera pass writes, given as an array to the occlusion call:
 most slots of the sphere's image hold none, and its rim is in every row, yet its
 neighbouring rays are alike and are traced as such."""
-import time
-
 import pytest
 
+import timing
 from gridrt import scenes
 
 pytestmark = pytest.mark.gpu
 
 
-def _best(call, runs=60):
-    """Seconds of the shortest of `runs` calls, each waited for."""
-    import torch
-    best = float("inf")
-    for _ in range(runs):
-        t = time.perf_counter()
-        call()
-        torch.cuda.synchronize()
-        best = min(best, time.perf_counter() - t)
-    return best
+def _pair(gridlib, verts, idx):
+    """The scene at one lane a ray, and the same with every 32 rays traced together."""
+    out = []
+    for refill in (None, 0):
+        s = gridlib.Scene(0)
+        s.set_geometry(verts, idx)
+        s.set_tuning(lanes=1, refill=refill)
+        s.build(4)
+        out.append(s)
+    return out
 
 
 @pytest.mark.parametrize("order", ["scanline", "morton8"])
@@ -31,22 +30,16 @@ def test_shadow_rays_of_an_image(gridlib, order):
     sc = scenes.deforming_sphere(3)
     cam = scenes.deforming_sphere_camera(640, 480)
     n = cam.width * cam.height
-    s = gridlib.Scene(0)
-    s.set_geometry(sc.verts, sc.idx)
-    s.set_tuning(lanes=1)
-    s.build(4)
+    s, whole = _pair(gridlib, sc.verts, sc.idx)
     hits = torch.zeros((n, 4), dtype=torch.int32, device="cuda")
     rays = torch.zeros((n, 8), dtype=torch.float32, device="cuda")
     s.trace_camera_device(cam, hits, scenes.SPHERE_LIGHT, rays, order=order)
     torch.cuda.synchronize()
     assert (rays[:, 7] < 0).float().mean() > 0.5
     got, want = torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.ones(n, dtype=torch.uint8, device="cuda")
-    as_set = _best(lambda: s.trace_any_device(rays, n, got))
-    s.set_tuning(refill=0)
-    together = _best(lambda: s.trace_any_device(rays, n, want))
+    slower = timing.ratio(lambda: s.trace_any_device(rays, n, got), lambda: whole.trace_any_device(rays, n, want), 1.15)
     assert torch.equal(got, want)
-    assert as_set < 1.15 * together, (as_set, together)
-    s.close()
+    assert slower < 1.15
 
 
 def test_camera_rays_whose_rows_end_inside_a_chunk(gridlib):
@@ -56,18 +49,13 @@ def test_camera_rays_whose_rows_end_inside_a_chunk(gridlib):
     import torch
     for lat in (24, 80):
         v, i, _ = scenes.sphere_mesh(lat, 2 * lat + 1)
-        s = gridlib.Scene(0)
-        s.set_geometry(v, i)
-        s.set_tuning(lanes=1)
-        s.build(4)
+        s, whole = _pair(gridlib, v, i)
         rays = torch.from_numpy(scenes.camera_rays(scenes.deforming_sphere_camera(540, 540))).cuda()
         got, want = (torch.full((len(rays), 4), x, dtype=torch.int32, device="cuda") for x in (7, 8))
-        as_set = _best(lambda: s.trace_nearest_device(rays, len(rays), got))
-        s.set_tuning(refill=0)
-        together = _best(lambda: s.trace_nearest_device(rays, len(rays), want))
+        slower = timing.ratio(lambda: s.trace_nearest_device(rays, len(rays), got),
+                              lambda: whole.trace_nearest_device(rays, len(rays), want), 1.12)
         assert torch.equal(got, want)
-        assert as_set < 1.12 * together, (lat, as_set, together)
-        s.close()
+        assert slower < 1.12, lat
 
 
 def test_shadow_rays_of_a_small_image(gridlib):
@@ -78,17 +66,11 @@ def test_shadow_rays_of_a_small_image(gridlib):
     sc = scenes.plane_and_debris(quads=35, debris=2550)
     cam = scenes.look_at_camera((0.0, 1.5, 3.0), (0.0, 0.3, 0.0), (0.0, 1.0, 0.0), 60.0, 512, 512)
     n = cam.width * cam.height
-    s = gridlib.Scene(0)
-    s.set_geometry(sc.verts, sc.idx)
-    s.set_tuning(lanes=1)
-    s.build(4)
+    s, whole = _pair(gridlib, sc.verts, sc.idx)
     hits = torch.zeros((n, 4), dtype=torch.int32, device="cuda")
     rays = torch.zeros((n, 8), dtype=torch.float32, device="cuda")
     s.trace_camera_device(cam, hits, scenes.PLANE_LIGHT, rays)
     got, want = torch.zeros(n, dtype=torch.uint8, device="cuda"), torch.ones(n, dtype=torch.uint8, device="cuda")
-    as_set = _best(lambda: s.trace_any_device(rays, n, got))
-    s.set_tuning(refill=0)
-    together = _best(lambda: s.trace_any_device(rays, n, want))
+    slower = timing.ratio(lambda: s.trace_any_device(rays, n, got), lambda: whole.trace_any_device(rays, n, want), 1.08)
     assert torch.equal(got, want)
-    assert as_set < 1.08 * together, (as_set, together)
-    s.close()
+    assert slower < 1.08
