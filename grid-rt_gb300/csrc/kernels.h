@@ -151,8 +151,8 @@ inline int refill_for(const TraceTuning& t, int mode_is_camera) {
 // occlusion and 7 for frames: in 5,000 triangles, several launches in flight,
 // 155,000 closest-hit rays take 81 us at 8 lanes and at one, 155,000 occlusion
 // segments 120 and 101; frames at 8 lanes and one, 512 x 512: plane and debris
-// 178 and 333, the sphere 120 and 129; 300 x 1,000, the sphere filling the
-// image: 193 and 151.
+// 178 and 333, the sphere 120 and 129 (image_lanes goes by what an image shows);
+// 300 x 1,000, the sphere filling the image: 193 and 151.
 inline int lanes_for(long long n, int sms, int quarters) {
     const long long resident = 1024LL * sms;
     if (8 * n <= resident) return 32;

@@ -289,9 +289,10 @@ __global__ void instances_prep_kernel(const InstanceRec* __restrict__ recs, int 
 }
 
 // Bound by the walks' latency and by the per-instance work of rays that miss:
-// 16 instances of three meshes, 1024^2 camera rays, 999 -> 660 us with the
-// sphere test (1,442 -> 947 us one launch at a time).  Six blocks of 128 an SM:
-// 736 / 673 / 660 / 644 us at 4 / 5 / 6 / 7, alone 986 / 939 / 947 / 969.
+// 16 instances of three meshes, 1024^2 camera rays, 1,073 -> 664 us with the
+// sphere test, three sets of instances in turn (997 -> 735 on another machine;
+// 1,442 -> 947 us one launch at a time).  Six blocks of 128 an SM: 736 / 673 /
+// 660 / 644 us at 4 / 5 / 6 / 7, alone 986 / 939 / 947 / 969.
 #ifndef GRIDRT_INST_MIN_BLOCKS
 #define GRIDRT_INST_MIN_BLOCKS 6
 #endif

@@ -39,8 +39,13 @@
 
 namespace gridrt {
 
-static constexpr float kChunkCells = 4.0f;   // chunk_alike: origins, in cells
-static constexpr float kChunkCone = 0.1f;    // and directions, of the first ray's length
+// chunk_alike: how far origins may be apart, in cells, and directions, in lengths
+// of the one compared with.  640 x 480 shadow rays of the sphere in Morton order:
+// 95 us at 4 and 8 cells, 119 at 2; its 1024^2 ones 128 at a cone of 0.02 to 0.1,
+// 162 at 0.01.  Against the first ray (tasks), 640 x 480 camera rays take 192 at
+// 0.1 and 235 at 0.05, 64 scenes in one batch 2,514 at 0.1 and 2,539 at 0.15.
+static constexpr float kChunkCells = 4.0f;
+static constexpr float kChunkCone = 0.1f;
 static constexpr unsigned FULL = 0xffffffffu;
 static constexpr int32_t kDeferred = -3;    // Lane::id of a ray handed to the group-of-lanes pass
 static constexpr int32_t kNoHeavy = 0x7fffffff;
