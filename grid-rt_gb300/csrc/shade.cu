@@ -304,12 +304,21 @@ rtg_status sfail(rtg_status s, const std::string& msg) {
 constexpr uint64_t kRenderKeep = 1ull << 30;
 
 std::mutex g_render_mutex;               // the list, and its scenes' render_kept
-std::vector<rtg_scene> g_rendered;       // scenes with a pool, least recently rendered first
+// Scenes with a pool, least recently rendered first (never destroyed: a scene may
+// go when the process does).
+std::vector<rtg_scene>& g_rendered = *new std::vector<rtg_scene>;
+
+// Another thread may be capturing: what the pools' upkeep calls does not touch
+// its streams.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 cudaMemPool_t render_pool(rtg_scene s) {
     std::call_once(s->render_once, [s] {
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // another thread may be capturing
-        cudaThreadExchangeStreamCaptureMode(&mode);
+        RelaxedCapture relaxed;
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
@@ -321,7 +330,6 @@ cudaMemPool_t render_pool(rtg_scene s) {
             s->render_pool = nullptr;   // frames use the default pool
             cudaGetLastError();
         }
-        cudaThreadExchangeStreamCaptureMode(&mode);
         if (s->render_pool) {
             std::lock_guard<std::mutex> lock(g_render_mutex);
             g_rendered.push_back(s);
@@ -333,6 +341,7 @@ cudaMemPool_t render_pool(rtg_scene s) {
 // After a frame: what the scene's pool keeps, and the bound on the device's.
 void keep_render_buffers(rtg_scene s) {
     if (!s->render_pool) return;
+    RelaxedCapture relaxed;
     std::lock_guard<std::mutex> lock(g_render_mutex);
     if (cudaMemPoolGetAttribute(s->render_pool, cudaMemPoolAttrReservedMemCurrent, &s->render_kept) != cudaSuccess)
         cudaGetLastError();
